@@ -7,92 +7,293 @@
 // sample covariance (N / (N - 1)), K1 = 0.01, K2 = 0.03, averaged over the
 // frame cropped by 3 pixels.  Every window of the cropped region lies inside
 // the frame, so the border extension of the uniform filter never enters the
-// mean.  A block stages a (TY + 6) x (TX + 6) tile of both frames in shared
-// memory; each thread forms its window's means, then the centred second
-// moments sum((x - mx)^2), sum((y - my)^2), sum((x - mx)(y - my)) (equal to
-// N (E[x^2] - mx^2) etc. without their cancellation), and the SSIM value;
-// per-block float64 partial sums go to per-frame float64 totals.  The same
-// pass sums (x - y)^2 over the whole frame for the PSNR.
+// mean.
+//
+// What bounds it.  Two frames are read once (8 bytes per pixel), 0.04 ms at
+// 2048 x 2048 x 8; the arithmetic of the windows is what costs.  With the
+// SSIM of a window in float64 (about 45 operations a pixel on a part that
+// does two float64 FMAs per clock and SM) and every window summed from
+// shared memory anew (196 loads a pixel) the pass took 3.5 ms.  Here:
+//
+//  * A warp owns a band of 128 columns (4 per lane) of one frame and marches
+//    down a chunk of rows with the last 7 rows in registers, so that a row
+//    is loaded once per band and window sums are separable: the moments of
+//    each 7-row column segment first, then of 7 neighbouring columns (6 of
+//    them shuffled in per lane of 4).
+//  * Moments are merged, not subtracted: sum (p - m)^2 of a column about its
+//    own mean, then sum over columns of those plus the spread of the column
+//    means.  No cancellation, so float32 keeps the accuracy of the direct
+//    two-pass sums.
+//  * The two moments needed are those of s = x + y and d = x - y, carried as
+//    one packed pair: with B1 = Mx^2 + My^2 + C1 and B2 = Vx + Vy + C2,
+//      SSIM = (1 - Md^2 / B1) (1 - Vd / B2),
+//      Mx^2 + My^2 = (Ms^2 + Md^2) / 2,  Vx + Vy = (Vs + Vd) / 2,
+//    so 1 - SSIM = e1 + e2 - e1 e2 is a sum of float32 quotients that are
+//    small where the images agree; its rounding is relative to 1 - SSIM.
+//  * Sums: the squared error of a pixel as an exact float32 product pair of
+//    an exact difference pair, and 1 - SSIM, are accumulated with
+//    compensated float32 additions over 8 rows and then added to float64.
+//
+// Measured at 2048 x 2048 x 8: 0.18 ms for the kernel (3.4 ms before), 58 %
+// of the issue slots; the packed float32 arithmetic of the windows bounds it
+// (about 100 instructions a pixel and lane, no spills at 3 blocks per SM; 4
+// blocks spill and take 0.20 ms).  Against float64, frames of 17 x 23 to
+// 2048 x 2048 with noise 0.003 to 0.1: mean SSIM at most 1.0e-8 off (2.4e-8
+// with float64 quotients of float32 moments), PSNR within 2e-14 dB.
+#include <algorithm>
+
 #include "sci_common.cuh"
 
 namespace sci {
 namespace {
 
-constexpr int TX = 32, TY = 8, R = 3, WIN = 2 * R + 1;
+constexpr int R = 3, WIN = 2 * R + 1;
+constexpr int WPB = 4;           // warps per block
+constexpr int BAND = 128;        // columns of a warp's window, 4 per lane
+constexpr int HALO = 4;          // its first and last columns, owned by the neighbours
+constexpr int OWN = BAND - 2 * HALO;
+constexpr int MIN_ROWS = 8;      // rows per chunk at least (6 more are read)
+constexpr int RESIDENT = 3;      // blocks per SM the registers are sized for
 
-__global__ void __launch_bounds__(TX * TY) k_frame_metrics(const float *__restrict__ a,
-                                                          const float *__restrict__ b, int H,
-                                                          int W, double C1, double C2,
-                                                          double *__restrict__ sqerr,
-                                                          double *__restrict__ ssim_sum) {
-    __shared__ float xa[TY + 2 * R][TX + 2 * R + 1], xb[TY + 2 * R][TX + 2 * R + 1];
-    __shared__ double red[2][TX * TY / 32];
-    const int64_t fo = (int64_t)blockIdx.z * H * W;
-    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;  // tile of window centres
-    const int tid = threadIdx.y * TX + threadIdx.x;
-    // stage the tile and its 3-pixel apron (clamped loads; clamped cells are
-    // only read by centres outside the cropped region, which are skipped)
-    for (int c = tid; c < (TY + 2 * R) * (TX + 2 * R); c += TX * TY) {
-        const int ly = c / (TX + 2 * R), lx = c - ly * (TX + 2 * R);
-        const int i = min(max(y0 + ly - R, 0), H - 1), j = min(max(x0 + lx - R, 0), W - 1);
-        xa[ly][lx] = a[fo + (int64_t)i * W + j];
-        xb[ly][lx] = b[fo + (int64_t)i * W + j];
+struct Metrics {
+    const float *a, *b;
+    double *sqerr, *ssim_sum;
+    int H, W, rows, nbands, nchunks;
+    int64_t items;
+    float scale;         // power of two near 1 / data_range: exact
+    double unscale2;     // 1 / scale^2
+    // 49^2 C1 and 7 48 C2 of the scaled frames, as pairs
+    float c1, c1_lo, c2, c2_lo;
+};
+
+// Sum of non-negative terms with its rounding errors: hi + lo.
+struct Comp {
+    float hi, lo;
+    __device__ __forceinline__ void add(float v, float v_lo) {
+        const float t = hi + v, z = t - hi;
+        lo += ((hi - (t - z)) + (v - z)) + v_lo;
+        hi = t;
     }
-    __syncthreads();
-    const int i = y0 + threadIdx.y, j = x0 + threadIdx.x;
-    double se = 0.0, ss = 0.0;
-    if (i < H && j < W) {
-        const double d = (double)xa[threadIdx.y + R][threadIdx.x + R] -
-                         (double)xb[threadIdx.y + R][threadIdx.x + R];
-        se = d * d;
-        if (i >= R && i < H - R && j >= R && j < W - R) {
-            float sx = 0.f, sy = 0.f;
+    // An infinite total has no rounding error (inf - inf is not one).
+    __device__ __forceinline__ double take() {
+        const double r = isfinite(hi) ? (double)hi + (double)lo : (double)hi;
+        hi = lo = 0.f;
+        return r;
+    }
+};
+
+// v / (h + c + c_lo).  The rounding of h + c goes into the reciprocal's
+// Newton step: left out, it has one sign for whole binades of h (c's last
+// bits are the same everywhere), a bias of the mean by up to 2^-25.
+__device__ __forceinline__ float quotient(float v, float h, float c, float c_lo) {
+    const float b = h + c, err = (c - (b - h)) + c_lo;
+    const float q = rcp_approx(b);
+    return v * fmaf(q, fmaf(-err, q, fmaf(-b, q, 1.f)), q);
+}
+
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float *p, int col, int W) {
+    if (VEC) return col < W ? ldg4(p + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(col < W ? __ldg(p + col) : 0.f, col + 1 < W ? __ldg(p + col + 1) : 0.f,
+                       col + 2 < W ? __ldg(p + col + 2) : 0.f,
+                       col + 3 < W ? __ldg(p + col + 3) : 0.f);
+}
+
+__device__ __forceinline__ f2 shfl_up2(f2 v) {
+    f2 r;
+    r.v = __shfl_up_sync(0xffffffffu, v.v, 1);
+    return r;
+}
+__device__ __forceinline__ f2 shfl_down2(f2 v) {
+    f2 r;
+    r.v = __shfl_down_sync(0xffffffffu, v.v, 1);
+    return r;
+}
+
+// VEC: rows are aligned for 16-byte loads (W % 4 == 0).
+template <bool VEC>
+__global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P) {
+    const int64_t item = (int64_t)blockIdx.x * WPB + (threadIdx.x >> 5);
+    if (item >= P.items) return;
+    const int lane = threadIdx.x & 31, H = P.H, W = P.W;
+    const int band = (int)(item % P.nbands);
+    const int64_t q = item / P.nbands;
+    const int chunk = (int)(q % P.nchunks);
+    const int64_t frame = q / P.nchunks;
+    const int c0 = band * OWN, col = c0 + 4 * lane;
+    const int own_lo = band == 0 ? 0 : c0 + HALO;
+    const int own_hi = band == P.nbands - 1 ? W : c0 + BAND - HALO;
+    const int r0 = chunk * P.rows, r1 = min(r0 + P.rows, H);
+    const int q0 = max(0, r0 - R), q1 = min(H, r1 + R);   // input rows
+    const int i0 = max(r0, R), i1 = min(r1, H - R);       // window centres
+    const float *pa = P.a + frame * H * W, *pb = P.b + frame * H * W;
+    // owned columns are whole lanes (own_lo, own_hi are multiples of 4, and
+    // columns past the frame read as 0 in both frames); the windows' are not
+    const bool own = col >= own_lo && col < own_hi;
+    float win[4];
+    int wins = 0;
 #pragma unroll
-            for (int u = 0; u < WIN; ++u)
+    for (int k = 0; k < 4; ++k) {
+        const bool w = own && col + k >= R && col + k < W - R;
+        win[k] = w ? 1.f : 0.f;
+        wins += w;
+    }
+
+    const f2 seventh = mk2(1.f / 7.f, 1.f / 7.f), seven = mk2(7.f, 7.f);
+    f2 p[WIN + 1][4];  // (s, d) of rows row - 6 .. row + 1
 #pragma unroll
-                for (int v = 0; v < WIN; ++v) {
-                    sx += xa[threadIdx.y + u][threadIdx.x + v];
-                    sy += xb[threadIdx.y + u][threadIdx.x + v];
-                }
-            const float mx = sx * (1.f / (WIN * WIN)), my = sy * (1.f / (WIN * WIN));
-            float vxx = 0.f, vyy = 0.f, vxy = 0.f;
+    for (int r = 0; r <= WIN; ++r)
 #pragma unroll
-            for (int u = 0; u < WIN; ++u)
+        for (int k = 0; k < 4; ++k) p[r][k].v = 0ull;
+    Comp se = {0.f, 0.f}, ds = {0.f, 0.f};
+    double sse = 0.0, dssim = 0.0;
+
+    // A new row: its (s, d) into slot q, its squared error into the sums.
+    auto take_row = [&](float4 va, float4 vb, f2 (&q)[4], bool count) {
+        const float x[4] = {va.x * P.scale, va.y * P.scale, va.z * P.scale, va.w * P.scale};
+        const float y[4] = {vb.x * P.scale, vb.y * P.scale, vb.z * P.scale, vb.w * P.scale};
 #pragma unroll
-                for (int v = 0; v < WIN; ++v) {
-                    const float dx = xa[threadIdx.y + u][threadIdx.x + v] - mx;
-                    const float dy = xb[threadIdx.y + u][threadIdx.x + v] - my;
-                    vxx = fmaf(dx, dx, vxx);
-                    vyy = fmaf(dy, dy, vyy);
-                    vxy = fmaf(dx, dy, vxy);
-                }
-            // sample covariance: divide by N - 1
-            const double inv = 1.0 / (WIN * WIN - 1);
-            const double Vx = vxx * inv, Vy = vyy * inv, Vxy = vxy * inv;
-            const double Mx = mx, My = my;
-            ss = ((2.0 * Mx * My + C1) * (2.0 * Vxy + C2)) /
-                 ((Mx * Mx + My * My + C1) * (Vx + Vy + C2));
+        for (int k = 0; k < 4; ++k) q[k] = mk2(x[k] + y[k], x[k] - y[k]);
+        if (!count) return;
+        // Squares whose rounding error float32 can hold: differences of 0
+        // or of 1e-12 to 1e18 (of the scaled frames).  Their bits less
+        // one, as unsigned, put 0 last; a vote, so that the float64 form
+        // is issued only where a difference is outside (or not a number).
+        unsigned most = 0u, least = ~0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned m = __float_as_uint(hi(q[k])) & 0x7fffffffu;
+            most = max(most, m);
+            least = min(least, m - 1u);
         }
+        const bool wide = most > __float_as_uint(1e18f) || least < __float_as_uint(1e-12f);
+        if (!__any_sync(0xffffffffu, wide)) {
+            // x - y = d + dl exactly; d^2 = t + its rounding error.  The
+            // products are scalar: ptxas contracts a packed product and a
+            // packed sum into an FMA, explicit rounding or not, and the
+            // error terms need the rounded product.
+            f2 t[2], e[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float d0 = hi(q[2 * h]), d1 = hi(q[2 * h + 1]);
+                const f2 X = mk2(x[2 * h], x[2 * h + 1]), Y = mk2(y[2 * h], y[2 * h + 1]);
+                const f2 d = mk2(d0, d1), z = sub2(d, X);
+                const f2 dl = sub2(sub2(X, sub2(d, z)), add2(Y, z));
+                t[h] = mk2(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
+                e[h] = fma2(add2(d, d), dl, fma2(d, d, sub2(mk2(0.f, 0.f), t[h])));
+            }
+            // t[0] + t[1], exactly as a sum and its error, then into the total
+            const f2 u = add2(t[0], t[1]), z = sub2(u, t[0]);
+            const f2 ue = add2(add2(sub2(t[0], sub2(u, z)), sub2(t[1], z)), add2(e[0], e[1]));
+            se.add(lo(u), lo(ue));
+            se.add(hi(u), hi(ue));
+        } else if (own) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double d = (double)x[k] - (double)y[k];
+                sse += d * d;
+            }
+        }
+    };
+    // The windows of one row of centres, from the sums of the common six
+    // rows and the seventh row `o`; held rows are p[1 .. 6] and o.
+    auto windows = [&](const f2 (&common)[4], const f2 (&o)[4]) {
+        f2 T[10], M[10];  // columns col - 3 .. col + 6: sum and centred sum of squares
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const f2 sum = add2(common[k], o[k]), mean = mul2(sum, seventh);
+            f2 c = sub2(o[k], mean), v = mul2(c, c);
+#pragma unroll
+            for (int r = 1; r < WIN; ++r) {
+                c = sub2(p[r][k], mean);
+                v = fma2(c, c, v);
+            }
+            T[k + 3] = sum;
+            M[k + 3] = v;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            T[k] = shfl_up2(T[k + 4]);
+            M[k] = shfl_up2(M[k + 4]);
+            T[k + 7] = shfl_down2(T[k + 3]);
+            M[k + 7] = shfl_down2(M[k + 3]);
+        }
+        // windows: columns k .. k + 6 of the ten, 3 .. 6 in all of them
+        const f2 Tc = add2(add2(T[3], T[4]), add2(T[5], T[6]));
+        const f2 Mc = add2(add2(M[3], M[4]), add2(M[5], M[6]));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            f2 S = Tc, V = Mc;
+#pragma unroll
+            for (int c = k; c < k + WIN; ++c)
+                if (c < 3 || c > 6) {
+                    S = add2(S, T[c]);
+                    V = add2(V, M[c]);
+                }
+            const f2 mean = mul2(S, seventh);  // of the column sums
+            f2 d = sub2(T[k], mean), w = mul2(d, d);
+#pragma unroll
+            for (int c = k + 1; c < k + WIN; ++c) {
+                d = sub2(T[c], mean);
+                w = fma2(d, d, w);
+            }
+            // e1 = Md^2 / B1 times 49^2 over 49^2, e2 = Vd / B2 times 7 48
+            // over 7 48, so that no factor is rounded
+            V = fma2(V, seven, w);
+            const f2 S2 = mul2(S, S);
+            const float e1 = quotient(hi(S2), 0.5f * (lo(S2) + hi(S2)), P.c1, P.c1_lo);
+            const float e2 = quotient(hi(V), 0.5f * (lo(V) + hi(V)), P.c2, P.c2_lo);
+            ds.add(fmaf(-e1, e2, e1 + e2) * win[k], 0.f);
+        }
+    };
+
+    float4 n0a = load4<VEC>(pa + (int64_t)q0 * W, col, W);
+    float4 n0b = load4<VEC>(pb + (int64_t)q0 * W, col, W);
+    float4 n1a = load4<VEC>(pa + (int64_t)(q0 + 1) * W, col, W);
+    float4 n1b = load4<VEC>(pb + (int64_t)(q0 + 1) * W, col, W);
+    // two rows at a time: the ring moves by register copies once per pair
+    // (48 of them; unrolling it away takes 7 copies of this body, more than
+    // the instruction cache holds)
+#pragma unroll 1
+    for (int row = q0; row < q1; row += 2) {
+        take_row(n0a, n0b, p[6], row >= r0 && row < r1);
+        take_row(n1a, n1b, p[7], row + 1 >= r0 && row + 1 < r1);
+        const int64_t next = (int64_t)min(row + 2, q1 - 1) * W, next1 = (int64_t)min(row + 3, q1 - 1) * W;
+        n0a = load4<VEC>(pa + next, col, W);
+        n0b = load4<VEC>(pb + next, col, W);
+        n1a = load4<VEC>(pa + next1, col, W);
+        n1b = load4<VEC>(pb + next1, col, W);
+        f2 common[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            common[k] = add2(add2(add2(p[1][k], p[2][k]), add2(p[3][k], p[4][k])),
+                             add2(p[5][k], p[6][k]));
+        const int i = row - R;  // centre of rows row - 6 .. row
+        if (i >= i0 && i < i1) windows(common, p[0]);
+        if (i + 1 >= i0 && i + 1 < i1) windows(common, p[7]);
+        if ((row & 6) == 6) {
+            const double a = se.take();
+            sse += own ? a : 0.0;
+            dssim += ds.take();
+        }
+#pragma unroll
+        for (int r = 0; r < WIN - 1; ++r)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) p[r][k] = p[r + 2][k];
     }
-    // block sums (fixed order within the block; float64 atomics across blocks)
+    const double a = se.take();
+    sse += own ? a : 0.0;
+    dssim += ds.take();
+    double ss = wins ? (double)wins * max(0, i1 - i0) - dssim : 0.0;
+    sse *= P.unscale2;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        se += __shfl_xor_sync(0xffffffffu, se, o);
+        sse += __shfl_xor_sync(0xffffffffu, sse, o);
         ss += __shfl_xor_sync(0xffffffffu, ss, o);
     }
-    if ((tid & 31) == 0) {
-        red[0][tid >> 5] = se;
-        red[1][tid >> 5] = ss;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double a0 = 0.0, a1 = 0.0;
-        for (int w = 0; w < TX * TY / 32; ++w) {
-            a0 += red[0][w];
-            a1 += red[1][w];
-        }
-        atomicAdd(sqerr + blockIdx.z, a0);
-        atomicAdd(ssim_sum + blockIdx.z, a1);
+    if (lane == 0) {
+        atomicAdd(P.sqerr + frame, sse);
+        atomicAdd(P.ssim_sum + frame, ss);
     }
 }
 
@@ -112,10 +313,38 @@ extern "C" int sci_frame_metrics(const float *orig, const float *x, int64_t nfra
     const cudaStream_t s = as_stream(stream);
     SCI_CUDA(cudaMemsetAsync(sqerr, 0, sizeof(double) * (size_t)nframes, s));
     SCI_CUDA(cudaMemsetAsync(ssim_sum, 0, sizeof(double) * (size_t)nframes, s));
-    const double C1 = (0.01 * data_range) * (0.01 * data_range);
-    const double C2 = (0.03 * data_range) * (0.03 * data_range);
-    const dim3 g((unsigned)((W + TX - 1) / TX), (unsigned)((H + TY - 1) / TY), (unsigned)nframes);
-    k_frame_metrics<<<g, dim3(TX, TY), 0, s>>>(orig, x, (int)H, (int)W, C1, C2, sqerr, ssim_sum);
+    Metrics P{};
+    P.a = orig;
+    P.b = x;
+    P.sqerr = sqerr;
+    P.ssim_sum = ssim_sum;
+    P.H = (int)H;
+    P.W = (int)W;
+    // frames scaled by a power of two to a data range in [1, 2)
+    const int e = std::max(-120, std::min(120, ilogb(data_range)));
+    P.scale = (float)ldexp(1.0, -e);
+    P.unscale2 = ldexp(1.0, 2 * e);
+    const double c1 = 2401.0 * (0.01 * data_range) * (0.01 * data_range) / P.unscale2;
+    const double c2 = 336.0 * (0.03 * data_range) * (0.03 * data_range) / P.unscale2;
+    P.c1 = (float)c1;
+    P.c1_lo = (float)(c1 - P.c1);
+    P.c2 = (float)c2;
+    P.c2_lo = (float)(c2 - P.c2);
+    // the bands' owned columns cover the frame: the last one's reach W
+    P.nbands = 1 + (int)std::max<int64_t>(0, (W - BAND + OWN - 1) / OWN);
+    // one wave of resident warps: a chunk of r rows reads r + 6, so taller
+    // chunks cost less as long as every warp slot has one
+    const int64_t cols = nframes * P.nbands, slots = (int64_t)kSMs * RESIDENT * WPB;
+    const int64_t most = (H + MIN_ROWS - 1) / MIN_ROWS;
+    P.nchunks = (int)std::max<int64_t>(1, std::min(most, slots / cols));
+    P.rows = (int)((H + P.nchunks - 1) / P.nchunks);
+    P.nchunks = (int)((H + P.rows - 1) / P.rows);
+    P.items = cols * P.nchunks;
+    const unsigned g = (unsigned)((P.items + WPB - 1) / WPB);
+    if (W % 4 == 0 && aligned16(orig) && aligned16(x))
+        k_frame_metrics<true><<<g, WPB * 32, 0, s>>>(P);
+    else
+        k_frame_metrics<false><<<g, WPB * 32, 0, s>>>(P);
     SCI_LAUNCHED("k_frame_metrics");
     return SCI_OK;
 }

@@ -187,6 +187,19 @@ static int choose_lag() {
     return 1;
 }
 
+// The register-tile pass (sci_tv_tile.cuh) where it is the faster one
+// (tile_wins).  SCI_TV_TILE=0 leaves every call to the row pipelines, 1 takes
+// tiles at every size; switches that shape the row pipelines (SCI_TV_SLIM=0,
+// SCI_TV_LAG, SCI_TV_R, SCI_TV_CPL, SCI_TV_ORDER, SCI_SLIM_MINB,
+// SCI_TV_FORM) leave it off too.
+static bool use_tiles(int64_t nf, int64_t H, int64_t W, bool slim) {
+    if (const char *e = getenv("SCI_TV_TILE")) return atoi(e) != 0;
+    for (const char *k : {"SCI_TV_LAG", "SCI_TV_R", "SCI_TV_CPL", "SCI_TV_ORDER",
+                          "SCI_SLIM_MINB", "SCI_TV_FORM"})
+        if (getenv(k)) return false;
+    return tv::tile_wins(nf, H, W, slim);
+}
+
 static int choose_cpl(int64_t W) {
     if (const char *e = getenv("SCI_TV_CPL")) {
         const int v = atoi(e);
@@ -294,6 +307,10 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
                      ((reinterpret_cast<uintptr_t>(f) | reinterpret_cast<uintptr_t>(u) |
                        reinterpret_cast<uintptr_t>(resid)) % (4 * cpl) == 0);
     const int minb = slim_minb(cpl);
+    // windows on tiles: any rule-0 call without a tape and without a row
+    // chunking or column width of the caller's; offsets in 32 bits
+    const bool tiles = slim_enabled() && ra.rule == RULE_SKIMAGE && !tape && force_R <= 0 &&
+                       fcpl == 0 && H * W < (int64_t(1) << 31) && use_tiles(nf, H, W, slim);
     const float *pin = nullptr;
     float *pbuf[2] = {w.pa, w.pb};
     int pi = 0;
@@ -357,7 +374,12 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
         P.ticket = stop_test ? w.ticket : nullptr;
         const int per_frame_blocks = (P.nbands * P.nchunks + WPB - 1) / WPB;
         P.gpf = std::max(1, std::min(per_frame_blocks, 16));
-        if (slim) {
+        if (tiles) {
+            const int c = tile_columns();
+            P.vec = aligned_for(c) && reinterpret_cast<uintptr_t>(ra.tout) % (4 * c) == 0;
+            tile_geometry(P);
+            launch_tile(P, PIN, FINAL, pmode, s);
+        } else if (slim) {
             launch_slim(P, SG, minb, pmode, s);
         } else if (tape) {
             launch_tape(P, SG, s);
@@ -378,7 +400,8 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
         }
         SCI_LAUNCHED("k_tv_main");
         if (stop_test) {
-            if (slim) launch_slim_fix(P, pmode, s);
+            if (tiles) launch_tile_fix(P, PIN, pmode, s);
+            else if (slim) launch_slim_fix(P, pmode, s);
             else if (proj) launch_fixup_proj(P, s);
             else launch_fixup(P, PIN, s);
             SCI_LAUNCHED("k_tv_fixup");

@@ -942,6 +942,11 @@ __global__ void __launch_bounds__(WPB * 32, min_blocks<CPL>()) k_tv_fixup(Pass P
 }
 
 // Host launchers (one translation unit each, compiled in parallel).
+bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim);  // sci_tv_tile.cu
+void tile_geometry(Pass &P);
+int tile_columns();
+void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s);
+void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s);
 void launch_main4_c4(const Pass &P, bool pin, bool final_pass, cudaStream_t s);
 void launch_main4_c2(const Pass &P, bool pin, bool final_pass, cudaStream_t s);
 void launch_main4_lag2(const Pass &P, bool pin, bool final_pass, cudaStream_t s);

@@ -193,3 +193,49 @@ def test_tv_slim_occupancy_variants(cpl, minbs, monkeypatch):
     for u, s, _ in outs[1:]:
         assert torch.equal(outs[0][0], u)
         assert list(outs[0][1]) == list(s)
+
+
+# The register-tile pass (sci_tv_tile.cuh: windows of 64 x 48 pixels, 56 x 40
+# owned; 2 x 8 pixels per thread) performs the row pipelines' operations in
+# their order, so frames are bit-identical and stop steps equal.  Sizes at
+# its edges: one pixel, frames smaller than a thread's rows, a window, its
+# halo; the frame's last row or column first or last in a window, a warp
+# (rows 8i) or a lane (odd widths); one to eight passes.
+TILE_SHAPES = [(1, 1, 2), (2, 3, 1), (5, 64, 2), (47, 63, 2), (48, 64, 3), (49, 65, 2), (44, 60, 1),
+               (45, 61, 1), (88, 120, 2), (89, 119, 2), (86, 121, 1), (125, 7, 3), (85, 175, 2),
+               (168, 176, 1), (130, 177, 3)]
+
+
+@pytest.mark.parametrize("H,W,F", TILE_SHAPES)
+@pytest.mark.parametrize("K", [2, 4, 5, 6, 9, 14, 30])
+def test_tv_tile_bitwise_equals_pipeline(H, W, F, K, monkeypatch):
+    fp = _dev.planar(smooth_frames(H, W, F, seed=H + 3 * W + K))
+    out = []
+    for tile in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        for eps in (2e-4, 0.02):  # the second stops most frames inside a pass
+            out.append(_tv_env(monkeypatch, fp, 0.1, K, eps, "1"))
+    for (u0, s0, e0), (u1, s1, e1) in zip(out[:2], out[2:]):
+        assert torch.equal(u0, u1)
+        assert list(s0) == list(s1)
+        # float32 sums of at most 16 terms per lane here, of a chunk's rows
+        # there; later passes of a stopped frame add nothing
+        np.testing.assert_allclose(e1, e0, rtol=1e-6, atol=1e-12)
+
+
+@pytest.mark.parametrize("H,W", [(50, 66), (97, 131)])
+def test_tv_tile_unaligned_and_resid(H, W, monkeypatch):
+    f = _dev.planar(smooth_frames(H, W, 2, seed=5))
+    store = torch.zeros(f.numel() + 1, device="cuda")
+    g = store[1:].view(f.shape)  # 4-byte aligned rows
+    g.copy_(f)
+    ref = None
+    for tile in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        for src in (f, g):
+            for K in (5, 11):
+                r = torch.full_like(f, 7.0)
+                u = sci.tv_frames(src, 0.2, K, resid=r)
+                assert torch.equal(r, u - f)
+                ref = ref or {}
+                assert torch.equal(ref.setdefault(K, u), u)

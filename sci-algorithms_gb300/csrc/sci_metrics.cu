@@ -30,9 +30,8 @@
 //      Mx^2 + My^2 = (Ms^2 + Md^2) / 2,  Vx + Vy = (Vs + Vd) / 2,
 //    so 1 - SSIM = e1 + e2 - e1 e2 is a sum of float32 quotients that are
 //    small where the images agree; its rounding is relative to 1 - SSIM.
-//  * Sums: the squared error of a pixel as an exact float32 product pair of
-//    an exact difference pair, and 1 - SSIM, are accumulated with
-//    compensated float32 additions over 8 rows and then added to float64.
+//  * Sums: the squared error (sci_sqerr.cuh) and 1 - SSIM are accumulated
+//    with compensated float32 additions over 8 rows and then added to float64.
 //
 // Measured at 2048 x 2048 x 8: 0.18 ms for the kernel (3.4 ms before), 58 %
 // of the issue slots; the packed float32 arithmetic of the windows bounds it
@@ -42,7 +41,7 @@
 // with float64 quotients of float32 moments), PSNR within 2e-14 dB.
 #include <algorithm>
 
-#include "sci_common.cuh"
+#include "sci_sqerr.cuh"
 
 namespace sci {
 namespace {
@@ -64,22 +63,6 @@ struct Metrics {
     double unscale2;     // 1 / scale^2
     // 49^2 C1 and 7 48 C2 of the scaled frames, as pairs
     float c1, c1_lo, c2, c2_lo;
-};
-
-// Sum of non-negative terms with its rounding errors: hi + lo.
-struct Comp {
-    float hi, lo;
-    __device__ __forceinline__ void add(float v, float v_lo) {
-        const float t = hi + v, z = t - hi;
-        lo += ((hi - (t - z)) + (v - z)) + v_lo;
-        hi = t;
-    }
-    // An infinite total has no rounding error (inf - inf is not one).
-    __device__ __forceinline__ double take() {
-        const double r = isfinite(hi) ? (double)hi + (double)lo : (double)hi;
-        hi = lo = 0.f;
-        return r;
-    }
 };
 
 // v / (h + c + c_lo).  The rounding of h + c goes into the reciprocal's
@@ -145,7 +128,9 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
     for (int r = 0; r <= WIN; ++r)
 #pragma unroll
         for (int k = 0; k < 4; ++k) p[r][k].v = 0ull;
-    Comp se = {0.f, 0.f}, ds = {0.f, 0.f};
+    SquareSum se;
+    se.clear();
+    Comp ds = {0.f, 0.f};
     double sse = 0.0, dssim = 0.0;
 
     // A new row: its (s, d) into slot q, its squared error into the sums.
@@ -154,45 +139,9 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
         const float y[4] = {vb.x * P.scale, vb.y * P.scale, vb.z * P.scale, vb.w * P.scale};
 #pragma unroll
         for (int k = 0; k < 4; ++k) q[k] = mk2(x[k] + y[k], x[k] - y[k]);
-        if (!count) return;
-        // Squares whose rounding error float32 can hold: differences of 0
-        // or of 1e-12 to 1e18 (of the scaled frames).  Their bits less
-        // one, as unsigned, put 0 last; a vote, so that the float64 form
-        // is issued only where a difference is outside (or not a number).
-        unsigned most = 0u, least = ~0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const unsigned m = __float_as_uint(hi(q[k])) & 0x7fffffffu;
-            most = max(most, m);
-            least = min(least, m - 1u);
-        }
-        const bool wide = most > __float_as_uint(1e18f) || least < __float_as_uint(1e-12f);
-        if (!__any_sync(0xffffffffu, wide)) {
-            // x - y = d + dl exactly; d^2 = t + its rounding error.  The
-            // products are scalar: ptxas contracts a packed product and a
-            // packed sum into an FMA, explicit rounding or not, and the
-            // error terms need the rounded product.
-            f2 t[2], e[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float d0 = hi(q[2 * h]), d1 = hi(q[2 * h + 1]);
-                const f2 X = mk2(x[2 * h], x[2 * h + 1]), Y = mk2(y[2 * h], y[2 * h + 1]);
-                const f2 d = mk2(d0, d1), z = sub2(d, X);
-                const f2 dl = sub2(sub2(X, sub2(d, z)), add2(Y, z));
-                t[h] = mk2(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-                e[h] = fma2(add2(d, d), dl, fma2(d, d, sub2(mk2(0.f, 0.f), t[h])));
-            }
-            // t[0] + t[1], exactly as a sum and its error, then into the total
-            const f2 u = add2(t[0], t[1]), z = sub2(u, t[0]);
-            const f2 ue = add2(add2(sub2(t[0], sub2(u, z)), sub2(t[1], z)), add2(e[0], e[1]));
-            se.add(lo(u), lo(ue));
-            se.add(hi(u), hi(ue));
-        } else if (own) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double d = (double)x[k] - (double)y[k];
-                sse += d * d;
-            }
+        if (count) {
+            const float d[4] = {hi(q[0]), hi(q[1]), hi(q[2]), hi(q[3])};
+            se.add4(x, y, d);
         }
     };
     // The windows of one row of centres, from the sums of the common six

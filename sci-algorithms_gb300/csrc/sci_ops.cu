@@ -11,7 +11,7 @@
 #include <cstring>
 #include <mutex>
 
-#include "sci_common.cuh"
+#include "sci_sqerr.cuh"
 
 namespace sci {
 
@@ -534,23 +534,50 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 }
 
 // ------------------------------------------------------- squared error
-__global__ void k_sqerr(const float *__restrict__ a, const float *__restrict__ b, int64_t n,
-                        double *out) {
+// *out += sum (a - b)^2, the PSNR numerator of an iteration.  Few blocks: each
+// ends in one float64 atomic on the same word, and 2048 of them, with two
+// conversions and two float64 operations per element, were 12 us of a 256 x
+// 256 x 8 iteration (3.0 now: 8 bytes per element, launch and reduction).
+// At 2048 x 2048 x 24 the float64 pipe bounded it at 0.60 ms; now 0.13 ms,
+// 6.2 TB/s of the 805 MB it reads.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_sqerr(const float *__restrict__ a,
+                                               const float *__restrict__ b, int64_t n,
+                                               double *out) {
+    grid_dep_wait();
+    SquareSum s;
+    s.clear();
     double acc = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double d = (double)a[i] - (double)b[i];
-        acc += d * d;
+    int turn = 0;
+    for (int64_t i = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
+         i += 4 * (int64_t)gridDim.x * blockDim.x) {
+        float x[4], y[4], d[4];
+        if (VEC) {
+            const float4 u = ldg4(a + i), v = ldg4(b + i);
+            x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
+            y[0] = v.x, y[1] = v.y, y[2] = v.z, y[3] = v.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                x[k] = i + k < n ? __ldg(a + i + k) : 0.f;
+                y[k] = i + k < n ? __ldg(b + i + k) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) d[k] = x[k] - y[k];
+        s.add4(x, y, d);
+        if ((++turn & 7) == 0) acc += s.take();
     }
+    acc += s.take();
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    __shared__ double red[32];
+    __shared__ double red[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) red[wid] = acc;
     __syncthreads();
-    if (wid == 0) {
-        acc = (lane < (int)(blockDim.x >> 5)) ? red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) atomicAdd(out, acc);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) acc += red[w];
+        atomicAdd(out, acc);
     }
 }
 
@@ -817,7 +844,13 @@ int sci_proj_admm(const float *theta, const float *b, const float *phi,
 int sci_sqerr_accum(const float *a, const float *b, int64_t n, double *out, void *stream) {
     SCI_CHECK_ARG(a && b && out && n >= 0, "sci_sqerr_accum: bad argument");
     if (n == 0) return SCI_OK;
-    k_sqerr<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(a, b, n, out);
+    // at least two groups of four per thread, at most four blocks per SM
+    const int64_t want = (n + 2047) / 2048, most = (int64_t)kSMs * 4;
+    const dim3 g((unsigned)(want < most ? want : most));
+    if (n % 4 == 0 && aligned16(a) && aligned16(b))
+        SCI_CUDA(launch_dep(k_sqerr<true>, g, dim3(256), 0, as_stream(stream), a, b, n, out));
+    else
+        SCI_CUDA(launch_dep(k_sqerr<false>, g, dim3(256), 0, as_stream(stream), a, b, n, out));
     SCI_LAUNCHED("k_sqerr");
     return SCI_OK;
 }

@@ -233,3 +233,23 @@ def test_proj_admm_matches_reference_step(packed):
          _dev.stream_handle())
     assert rel(_dev.unplanar(xo, th), xr) < RTOL
     assert rel(_dev.unplanar(v, th), xr - b) < RTOL
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 2047, 2048, 2052, 152 * 4 * 2048 + 5, 152 * 4 * 2048 * 9])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sqerr_accum_is_exact_to_float64(n, offset):
+    # sums of exact squares (products and differences as float32 pairs): the
+    # pairs hold 2^-45 of a term; offset 1: 4-byte aligned pointers
+    from sci_algorithms_gb300._lib import call
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.rand(n + offset, device="cuda", generator=g)[offset:]
+    b = torch.rand(n + offset, device="cuda", generator=g)[offset:]
+    for scale in (1.0, 1e-15, 1e15):  # the middle one in the float64 branch
+        x, y = (t * scale for t in (a, b))
+        if offset:  # the products above are aligned copies
+            x, y = (torch.cat([t[:1], t])[1:] for t in (x, y))
+        out = torch.full((1,), 2.0 * scale * scale, dtype=torch.float64, device="cuda")
+        call("sci_sqerr_accum", x.data_ptr(), y.data_ptr(), n, out.data_ptr(),
+             torch.cuda.current_stream().cuda_stream)
+        ref = 2.0 * scale * scale + ((x.double() - y.double()) ** 2).sum().item()
+        assert abs(out.item() / ref - 1) < 1e-12

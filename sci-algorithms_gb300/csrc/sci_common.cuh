@@ -67,6 +67,13 @@ cudaError_t launch_dep(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem,
 __device__ __forceinline__ void grid_dep_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Lets the next kernel's blocks be scheduled once every block of this grid
+// has started: as the last wave drains, they take the freed slots (and wait).
+// For grids of more than one wave; blocks that wait beside a grid that is
+// resident as a whole gain nothing.  Call after grid_dep_wait().
+__device__ __forceinline__ void grid_dep_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ------------------------------------------------------------- device side
 __device__ __forceinline__ float4 ldg4(const float *p) {

@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
     float *__restrict__ y1, const float *__restrict__ phisum, float *__restrict__ c, int B,
     int64_t hw, double *__restrict__ rn, double *__restrict__ zero, int nzero, int rev) {
     grid_dep_wait();
+    if (gridDim.x > kSMs * 8) grid_dep_launch();
     if (blockIdx.x == 0)  // the next TV pass's stop-test sums
         for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0.0;
     const int64_t n4 = hw >> 2;
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
     float gamma, int B, int64_t hw, double *__restrict__ rn, double *__restrict__ zero,
     int nzero, int rev) {
     grid_dep_wait();
+    if (gridDim.x > kSMs * 8) grid_dep_launch();
     if (blockIdx.x == 0)  // the next TV pass's stop-test sums
         for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0.0;
     auto tload = [&](int64_t o) {

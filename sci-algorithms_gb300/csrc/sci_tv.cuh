@@ -104,6 +104,7 @@ struct Pass {
     // Lean pass with the projection on load and the t output (PROJ 3):
     // t = u + (u - f) of every frame, same layout as u (nullable otherwise).
     float *tout;
+    int early;            // more blocks than fit at once: grid_dep_launch()
 };
 
 // Dual update rules of the pipeline (the dual p is held as p / lambda for
@@ -945,6 +946,8 @@ __global__ void __launch_bounds__(WPB * 32, min_blocks<CPL>()) k_tv_fixup(Pass P
 bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim);  // sci_tv_tile.cu
 void tile_geometry(Pass &P);
 int tile_columns();
+int64_t tile_blocks(const Pass &P);
+int tile_resident_blocks();
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s);
 void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s);
 void launch_main4_c4(const Pass &P, bool pin, bool final_pass, cudaStream_t s);

@@ -15,7 +15,7 @@ namespace tv {
 namespace {
 constexpr int C = 2, N = 4, NW = 6, MINB = 4;
 
-dim3 blocks(const Pass &P) { return dim3((unsigned)((int64_t)P.nbands * P.nchunks * P.nf)); }
+dim3 blocks(const Pass &P) { return dim3((unsigned)tile_blocks(P)); }
 
 template <bool PIN, bool OUT_U, int PROJ>
 void main_pass(const Pass &P, cudaStream_t s) {
@@ -55,6 +55,8 @@ void tile_geometry(Pass &P) {
     P.nbands = tile::window_count(P.W, G::COLS);
 }
 int tile_columns() { return C; }
+int64_t tile_blocks(const Pass &P) { return (int64_t)P.nbands * P.nchunks * P.nf; }
+int tile_resident_blocks() { return MINB; }
 
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s) {
     if (proj == 3) main_pass<false, true, 3>(P, s);

@@ -392,6 +392,7 @@ template <int C, int N, int NW, int MINB, bool PIN, bool OUT_U, int PROJ>
 __global__ void __launch_bounds__(NW * 32, MINB) k_tv_tile(Pass P) {
     __shared__ Smem<C, NW> sm;
     grid_dep_wait();
+    if (P.early) grid_dep_launch();
     int frame, tr, tc;
     decode(P, frame, tr, tc);
     if (!(PIN && P.done[frame] >= 0))  // not stopped in an earlier pass
@@ -407,6 +408,7 @@ template <int C, int N, int NW, int MINB, bool PIN, int PROJ>
 __global__ void __launch_bounds__(NW * 32, MINB) k_tv_tile_fix(Pass P) {
     __shared__ Smem<C, NW> sm;
     grid_dep_wait();
+    if (P.early) grid_dep_launch();
     int frame, tr, tc;
     decode(P, frame, tr, tc);
     const int j = P.stopj[frame];

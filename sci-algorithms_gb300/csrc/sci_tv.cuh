@@ -90,9 +90,9 @@ struct Pass {
     // the anisotropic Chambolle projection (RULE_CHAM_ITV) or the clip
     // bound (RULE_CLIP); c2 scales div p in u = f - c2 div p (RULE_CLIP)
     float c1, c2;
-    // Tape of a single-pass run (kernels with TAPE = true): every stage k
-    // writes its p_k to tape_p [S][nf][2][H][W] and, for k < S, its u_k to
-    // tape_u [S-1][nf][H][W] (the reverse pass of the unrolled solver).
+    // Tape of a single-pass run on tiles (sci_tv_tile.cuh, TAPE): 4 p_k of every
+    // update k = 1..S in tape_p [S][nf][2][H][W], u_k (k < S) in tape_u
+    // [S-1][nf][H][W] (the reverse pass of the unrolled solver).
     float *tape_p, *tape_u;
     // Stop decisions of the pass (nullable; kernels with energies): the
     // main launch's last block to finish writes stopj[frame] = the stop
@@ -105,6 +105,10 @@ struct Pass {
     // t = u + (u - f) of every frame, same layout as u (nullable otherwise).
     float *tout;
     int early;            // more blocks than fit at once: grid_dep_launch()
+    // Unrolled solver (sci_tv_tile.cuh, PROJ 2): frames are frames frame0 ..
+    // of N scenes of B; f holds x, cmap the scenes' maps q, phi [B][H][W].
+    const float *phi, *lam_dev;
+    int frame0, B;
 };
 
 // Dual update rules of the pipeline (the dual p is held as p / lambda for
@@ -276,7 +280,7 @@ __device__ __forceinline__ Row<CPL> divergence(const Row<CPL> &prn, const Row<CP
 // One pipeline step: input row r enters, stage k handles row r-k.
 // GEN: rows may be outside [r0, r1) or touch the frame's first/last row.
 template <int S, int CPL, bool PIN, bool OUT_U, bool ENERGY, int MODE, bool GEN, int PROJ,
-          int RULE = RULE_SKIMAGE, bool TAPE = false>
+          int RULE = RULE_SKIMAGE>
 __device__ __forceinline__ void step(const Pass &P, const St<S, CPL> &in, St<S, CPL> &out,
                                      int r, int rs, int r0, int r1, const Lane<CPL> &L,
                                      const float *fb, const float *pinb, float *ob, float *rb,
@@ -410,16 +414,6 @@ __device__ __forceinline__ void step(const Pass &P, const St<S, CPL> &in, St<S, 
                 }
             }
         }
-        if (TAPE && (!GEN || (i >= r0 && i < r1))) {
-            const int64_t ro = (int64_t)i * W;
-            float *tp = P.tape_p + ((int64_t)(k - 1) * P.nf + frame) * 2 * hw;
-            store_row<CPL, MODE>(tp + ro, L.col, prn, L.lane_own, L.mk, vec);
-            store_row<CPL, MODE>(tp + hw + ro, L.col, pcn, L.lane_own, L.mk, vec);
-            if (k < S) {
-                float *tu = P.tape_u + ((int64_t)(k - 1) * P.nf + frame) * hw;
-                store_row<CPL, MODE>(tu + ro, L.col, uk, L.lane_own, L.mk, vec);
-            }
-        }
         if (k == S) {
             if (!GEN || (i >= r0 && i < r1)) {
                 const int64_t ro = (int64_t)i * W;
@@ -484,7 +478,7 @@ __device__ __forceinline__ bool band_interior(const Pass &P, int c0, int width) 
 }
 
 template <int S, int CPL, bool PIN, bool OUT_U, bool ENERGY, int MODE, int PROJ,
-          int RULE = RULE_SKIMAGE, bool TAPE = false, bool RES = true>
+          int RULE = RULE_SKIMAGE, bool RES = true>
 __device__ __forceinline__ void run(const Pass &P, int frame, int chunk, int band, int lane) {
     const int H = P.H, W = P.W;
     Lane<CPL> L;
@@ -533,15 +527,15 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int chunk, int ban
     while (r <= rlast) {
         if (r == rfb && r + 1 <= rfe) {
             for (; r + 1 <= rfe; r += 2) {
-                step<S, CPL, PIN, OUT_U, ENERGY, MODE, false, PROJ, RULE, TAPE>(
+                step<S, CPL, PIN, OUT_U, ENERGY, MODE, false, PROJ, RULE>(
                     P, A, B, r, rs, r0, r1, L, fb, pinb, ob, rb, ek, frame);
-                step<S, CPL, PIN, OUT_U, ENERGY, MODE, false, PROJ, RULE, TAPE>(
+                step<S, CPL, PIN, OUT_U, ENERGY, MODE, false, PROJ, RULE>(
                     P, B, A, r + 1, rs, r0, r1, L, fb, pinb, ob, rb, ek, frame);
             }
             continue;
         }
         // prologue (halo rows, first S steps) and epilogue (chunk tail, last row)
-        step<S, CPL, PIN, OUT_U, ENERGY, MODE, true, PROJ, RULE, TAPE>(P, A, B, r, rs, r0, r1, L,
+        step<S, CPL, PIN, OUT_U, ENERGY, MODE, true, PROJ, RULE>(P, A, B, r, rs, r0, r1, L,
                                                                         fb, pinb, ob, rb, ek,
                                                                         frame);
         A = B;
@@ -799,21 +793,20 @@ __device__ __forceinline__ void run2(const Pass &P, int frame, int chunk, int ba
 }
 
 template <int S, int CPL, bool PIN, bool OUT_U, bool ENERGY, int LAG = 1, int PROJ = 0,
-          int RULE = RULE_SKIMAGE, bool TAPE = false, bool RES = true>
+          int RULE = RULE_SKIMAGE, bool RES = true>
 __device__ __forceinline__ void run_mode(const Pass &P, int frame, int chunk, int band, int lane) {
     int c0, lo, hi;
     band_window(P, band, 32 * CPL, c0, lo, hi);
     const bool interior = P.vec && band_interior(P, c0, 32 * CPL);
-    static_assert(!(TAPE && LAG == 2), "the tape is written by the lag-1 pipeline");
     if (LAG == 2) {
         if (interior) run2<S, CPL, PIN, OUT_U, ENERGY, INTERIOR>(P, frame, chunk, band, lane);
         else run2<S, CPL, PIN, OUT_U, ENERGY, EDGE>(P, frame, chunk, band, lane);
     } else {
         if (interior)
-            run<S, CPL, PIN, OUT_U, ENERGY, INTERIOR, PROJ, RULE, TAPE, RES>(P, frame, chunk,
+            run<S, CPL, PIN, OUT_U, ENERGY, INTERIOR, PROJ, RULE, RES>(P, frame, chunk,
                                                                               band, lane);
         else
-            run<S, CPL, PIN, OUT_U, ENERGY, EDGE, PROJ, RULE, TAPE, RES>(P, frame, chunk, band,
+            run<S, CPL, PIN, OUT_U, ENERGY, EDGE, PROJ, RULE, RES>(P, frame, chunk, band,
                                                                           lane);
     }
 }
@@ -889,15 +882,15 @@ __device__ __forceinline__ void decide_stops(const Pass &P, int lane) {
 
 // Main launch of one pass: every frame not yet stopped runs all SG updates.
 template <int SG, bool PIN, bool FINAL, int CPL, int LAG = 1, int PROJ = 0,
-          int RULE = RULE_SKIMAGE, bool TAPE = false, bool RES = true>
+          int RULE = RULE_SKIMAGE, bool RES = true>
 __global__ void __launch_bounds__(WPB * 32, min_blocks<CPL>()) k_tv_main(Pass P) {
     int frame, chunk, band;
     if (!decode_item(P, frame, chunk, band)) return;
-    // the MATLAB rules and the taped runs have no stop test and need no energies
-    constexpr bool EN = RULE == RULE_SKIMAGE && !TAPE;
+    // the MATLAB rules have no stop test and need no energies
+    constexpr bool EN = RULE == RULE_SKIMAGE;
     const int lane = threadIdx.x & 31;
     if (!(PIN && P.done[frame] >= 0))  // not stopped in an earlier pass
-        run_mode<SG, CPL, PIN, FINAL, EN, LAG, PROJ, RULE, TAPE, RES>(P, frame, chunk, band,
+        run_mode<SG, CPL, PIN, FINAL, EN, LAG, PROJ, RULE, RES>(P, frame, chunk, band,
                                                                       lane);
     if constexpr (EN) {
         if (P.ticket) decide_stops(P, lane);
@@ -956,7 +949,6 @@ void launch_main4_lag2(const Pass &P, bool pin, bool final_pass, cudaStream_t s)
 void launch_main_proj(const Pass &P, int SG, cudaStream_t s);
 void launch_fixup_proj(const Pass &P, cudaStream_t s);
 void launch_main123(const Pass &P, int SG, bool pin, cudaStream_t s);
-void launch_tape(const Pass &P, int SG, cudaStream_t s);  // sci_tv_tape.cu
 void launch_rule1(const Pass &P, int SG, bool pin, bool final_pass, cudaStream_t s);
 void launch_rule2(const Pass &P, int SG, bool pin, bool final_pass, cudaStream_t s);
 void launch_rule3(const Pass &P, int SG, bool pin, bool final_pass, cudaStream_t s);

@@ -33,6 +33,8 @@
 //    shorter update count rewrites the frames that stop (k_tv_tile_fix).
 #pragma once
 
+#include <type_traits>
+
 #include "sci_tv.cuh"
 
 namespace sci {
@@ -62,49 +64,143 @@ __device__ __forceinline__ void window(int n, int width, int i, int count, int &
 }
 
 // How a window's rows are read and written: aligned vectors of a window
-// inside the frame; aligned vectors with bounds; scalars with bounds.
-enum { INSIDE = 0, EDGE_VEC = 1, EDGE_SCALAR = 2 };
+// inside the frame; aligned vectors with bounds; scalars with bounds; the same
+// where a window's rows span 4 GB or more.
+enum { INSIDE = 0, EDGE_VEC = 1, EDGE_SCALAR = 2, EDGE_WIDE = 3 };
 
-// C consecutive values of a plane at offset `o` (its row inside the frame;
-// row_in: so it is), columns col ..; cells outside read as 0.  No branches:
-// the callers clamp the row, the value is selected.
-template <int C, int MODE>
-__device__ __forceinline__ void load_cols(const float *__restrict__ plane, unsigned o, int col,
-                                          int W, bool row_in, float (&v)[C]) {
-    if (MODE == EDGE_SCALAR) {
+// Where a thread's rows lie in every plane of a frame: a base per window (the
+// same for the block) and a byte offset per row, formed once, so that a load
+// or store costs one addition.  Offsets are 32 bits but for EDGE_WIDE.  Rows
+// and columns outside the frame are clamped into it and their
+// values replaced by 0.
+template <int C, int N, int MODE>
+struct Cells {
+    static constexpr bool SCALAR = MODE >= EDGE_SCALAR;
+    using Off = typename std::conditional<MODE == EDGE_WIDE, int64_t, unsigned>::type;
+    int64_t base;    // element offset of the window's row max(t0 - 1, 0)
+    Off off[2][N];   // rows row + j + h N
+    int rows, cols;  // of the thread's cells, how many lie inside the frame
+    unsigned step;   // scalars: bytes to the second column (0 outside)
+
+    __device__ __forceinline__ Off at(int r, int col, int tb, int H, int W) const {
+        const int c = SCALAR ? min(col, W - 1) : (MODE == INSIDE ? col : min(col, W - C));
+        return ((Off)((MODE == INSIDE ? r : min(r, H - 1)) - tb) * (Off)W + (Off)c) * 4;
+    }
+    __device__ __forceinline__ Cells(int t0, int row, int col, int H, int W) {
+        const int tb = max(t0 - 1, 0);
+        base = (int64_t)tb * W;
+        rows = H - row;
+        cols = W - col;
+        step = cols > 1 ? 4u : 0u;
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-            const float t = __ldg(plane + (o + min(col + c, W - 1)));
-            v[c] = row_in && col + c < W ? t : 0.f;
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                off[h][j] = MODE == INSIDE ? at(row, col, tb, H, W) + (Off)(j + h * N) * (Off)W * 4
+                                           : at(row + j + h * N, col, tb, H, W);
+    }
+    // Plain loads, not the read-only path: with programmatic launches the
+    // rows may be written by the kernel before while this one's blocks
+    // already wait.
+    __device__ __forceinline__ void load(const float *plane, Off o, bool row_in,
+                                         float (&v)[C]) const {
+        const char *p = reinterpret_cast<const char *>(plane + base), *q = p + o;
+        if (SCALAR) {
+            static_assert(!SCALAR || C == 2, "scalars: two columns");
+            // in this order: the two loads touch the same sectors, and a row's
+            // lines leave L1 before a second sweep over the rows
+            float a, b;
+            asm volatile("ld.global.f32 %0, [%1];" : "=f"(a) : "l"(q));
+            asm volatile("ld.global.f32 %0, [%1];" : "=f"(b) : "l"(p + (Off)(o + step)));
+            v[0] = row_in && cols > 0 ? a : 0.f;
+            v[C - 1] = row_in && cols > 1 ? b : 0.f;
+            return;
         }
-        return;
-    }
-    const float *q = plane + (o + (MODE == INSIDE ? col : min(col, W - C)));
-    if constexpr (C == 4) {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(q));
-        v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-    } else {
-        const float2 t = __ldg(reinterpret_cast<const float2 *>(q));
-        v[0] = t.x, v[1] = t.y;
-    }
-    if (MODE != INSIDE) {
-        const bool in = row_in && col < W;
+        if constexpr (C == 4) {
+            const float4 t = *reinterpret_cast<const float4 *>(q);
+            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+        } else {
+            const float2 t = *reinterpret_cast<const float2 *>(q);
+            v[0] = t.x, v[1] = t.y;
+        }
+        if (MODE != INSIDE) {
 #pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = in ? v[c] : 0.f;
+            for (int c = 0; c < C; ++c) v[c] = row_in && cols > 0 ? v[c] : 0.f;
+        }
     }
-}
+    __device__ __forceinline__ bool inside(int h, int j) const {
+        return MODE == INSIDE || j + h * N < rows;
+    }
+    __device__ __forceinline__ void load(const float *plane, int h, int j, float (&v)[C]) const {
+        load(plane, off[h][j], inside(h, j), v);
+    }
+    // the thread's rows of a plane as pairs
+    __device__ __forceinline__ void load(const float *plane, f2 (&v)[N][C]) const {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            float a[2][C];
+            load(plane, 0, j, a[0]);
+            load(plane, 1, j, a[1]);
+#pragma unroll
+            for (int c = 0; c < C; ++c) v[j][c] = mk2(a[0][c], a[1][c]);
+        }
+    }
+    // its upper and lower N rows of a plane, where `top`, `bottom` say that
+    // the window owns them
+    __device__ __forceinline__ void store(float *plane, const f2 (&v)[N][C], bool top,
+                                          bool bottom) const {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!(h ? bottom : top)) continue;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                if (!inside(h, j)) break;
+                float *q = reinterpret_cast<float *>(reinterpret_cast<char *>(plane + base) +
+                                                     off[h][j]);
+                float a[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) a[c] = h ? hi(v[j][c]) : lo(v[j][c]);
+                if (SCALAR) {
+#pragma unroll
+                    for (int c = 0; c < C; ++c)
+                        if (c < cols) q[c] = a[c];
+                } else if constexpr (C == 4) {
+                    *reinterpret_cast<float4 *>(q) = make_float4(a[0], a[1], a[2], a[3]);
+                } else {
+                    *reinterpret_cast<float2 *>(q) = make_float2(a[0], a[1]);
+                }
+            }
+        }
+    }
+};
 
-// Columns of a lane that owns them (n: how many lie inside the frame).
-template <int C, int MODE>
-__device__ __forceinline__ void store_cols(float *q, int n, const float (&v)[C]) {
-    if (MODE == EDGE_SCALAR) {
+// One row of the input f of a frame (its stack at fb): the stored values, or
+// with the projection applied as it is loaded -- PROJ 1, 3: a packed binary
+// mask (proj_px); PROJ 2: the unrolled solver's v = x + lam (q phi_b), with a
+// float mask per frame of a scene, the map q per scene and lam in device
+// memory.
+template <int PROJ, int C, int N, int MODE, typename Args>
+__device__ __forceinline__ void load_f(const Args &P, const Cells<C, N, MODE> &X,
+                                       const float *fb, int frame,
+                                       typename Cells<C, N, MODE>::Off o, bool in,
+                                       float (&v)[C]) {
+    X.load(fb, o, in, v);
+    if constexpr (PROJ == 1 || PROJ == 3) {
+        float cm[C], wb[C];
+        X.load(P.cmap, o, in, cm);
+        X.load(reinterpret_cast<const float *>(P.bits), o, in, wb);
 #pragma unroll
         for (int c = 0; c < C; ++c)
-            if (c < n) q[c] = v[c];
-    } else if constexpr (C == 4) {
-        *reinterpret_cast<float4 *>(q) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-        *reinterpret_cast<float2 *>(q) = make_float2(v[0], v[1]);
+            v[c] = proj_px(P.lam, cm[c], v[c], __float_as_uint(wb[c]), 1u << frame);
+    } else if constexpr (PROJ == 2) {
+        const int64_t hw = (int64_t)P.H * P.W;
+        const int g = P.frame0 + frame, n = g / P.B;
+        float q[C], m[C];
+        X.load(P.cmap + n * hw, o, in, q);
+        X.load(P.phi + (g - n * P.B) * hw, o, in, m);
+        const float lam = *P.lam_dev;
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = fmaf(lam, q[c] * m[c], v[c]);
     }
 }
 
@@ -151,8 +247,9 @@ struct Smem {
 // The window of one block: nup dual updates (nup <= SMAX) of tile (tr, tc)
 // of `frame`.  PIN: start from p_a (P.p_in).  OUT_U: write u (and resid,
 // with PROJ 3 t = u + (u - f)), else p (P.p_out).  ENERGY: add the pass's
-// energy sums.  EDGE: the window touches a frame edge.
-template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ, int MODE>
+// energy sums.  TAPE: also write every p_k (as 4 p) and, for k < nup, u_k
+// (P.tape_p, P.tape_u).  EDGE: the window touches a frame edge.
+template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ, bool TAPE, int MODE>
 __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, int nup,
                                     Smem<C, NW> &sm) {
     using G = Geo<C, N, NW>;
@@ -165,6 +262,13 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
     const int col = c0 + C * lane, row = t0 + 2 * N * w;  // this thread's first
     const int64_t hw = (int64_t)H * W;
     const float *fb = P.f + (int64_t)frame * P.fs;
+    // halves of a thread's rows are owned or not, up to the frame's last row
+    static_assert(HALO % N == 0 && HALO % C == 0, "window edges split no half and no lane");
+    const bool cols = col >= own_c0 && col < own_c1;
+    const bool top = cols && row >= own_r0 && row < own_r1;
+    const bool bottom = cols && row + N >= own_r0 && row + N < own_r1;
+    const Cells<C, N, MODE> X(t0, row, col, H, W);
+    auto store = [&](float *plane, const f2 (&v)[N][C]) { X.store(plane, v, top, bottom); };
 
     f2 f[N][C], u[N][C], pr[N][C], pc[N][C];
     // ---- input rows
@@ -173,18 +277,7 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
         float v[2][C];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int r = row + j + h * N;
-            const bool in = !EDGE || r < H;
-            const unsigned o = (unsigned)(EDGE ? min(r, H - 1) : r) * (unsigned)W;
-            load_cols<C, MODE>(fb, o, col, W, in, v[h]);
-            if (PROJ) {  // f = x + lam (c phi_b), as the GAP projection rounds it
-                float cm[C], wb[C];
-                load_cols<C, MODE>(P.cmap, o, col, W, in, cm);
-                load_cols<C, MODE>(reinterpret_cast<const float *>(P.bits), o, col, W, in, wb);
-#pragma unroll
-                for (int c = 0; c < C; ++c)
-                    v[h][c] = proj_px(P.lam, cm[c], v[h][c], __float_as_uint(wb[c]), 1u << frame);
-            }
+            load_f<PROJ>(P, X, fb, frame, X.off[h][j], X.inside(h, j), v[h]);
         }
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -228,21 +321,17 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
         const float *pb = P.p_in + (int64_t)frame * 2 * hw;
         float above[C];
         f2 left0[N];
-        load_cols<C, MODE>(pb, (unsigned)min(max(row - 1, 0), H - 1) * (unsigned)W, col, W, true,
-                           above);
-#pragma unroll
-        for (int c = 0; c < C; ++c) above[c] = row > 0 ? above[c] : 0.f;
+        X.load(pb, X.at(max(row - 1, 0), col, max(t0 - 1, 0), H, W), row > 0, above);
+        const unsigned lo0 = (unsigned)max(c0 - 1, 0);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             float a[2][C], b[2][C], l[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+                X.load(pb, h, j, a[h]);
+                X.load(pb + hw, h, j, b[h]);
                 const int r = row + j + h * N;
-                const bool in = !EDGE || r < H;
-                const unsigned o = (unsigned)(EDGE ? min(r, H - 1) : r) * (unsigned)W;
-                load_cols<C, MODE>(pb, o, col, W, in, a[h]);
-                load_cols<C, MODE>(pb + hw, o, col, W, in, b[h]);
-                const float t = __ldg(pb + hw + (o + max(c0 - 1, 0)));
+                const float t = pb[hw + ((unsigned)min(r, H - 1) * (unsigned)W + lo0)];
                 l[h] = c0 > 0 && r < H ? t : 0.f;
             }
 #pragma unroll
@@ -293,6 +382,11 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
                 if (ENERGY) ek[k - 1] = fma2(w2, n, ek[k - 1]);
             }
         }
+        if (TAPE) {
+            float *tp = P.tape_p + ((int64_t)(k - 1) * P.nf + frame) * 2 * hw;
+            store(tp, pr);
+            store(tp + hw, pc);
+        }
         if (!OUT_U && k == nup) break;  // p alone goes on
         // ---- u_k = f - div p_k / 4
         float last[C], above[C];
@@ -304,49 +398,28 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
         for (int c = 0; c < C; ++c) above[c] = 0.f;
         if (w > 0) sm.p.get(w - 1, lane, above);
         divergence(above, zero_left, k < SMAX && k < nup, ek[k < SMAX ? k : 0]);
+        if (TAPE && k < nup) store(P.tape_u + ((int64_t)(k - 1) * P.nf + frame) * hw, u);
     }
 
-    // ---- owned rows out (halves of a thread's rows are owned or not, up to
-    // the frame's last row)
-    static_assert(HALO % N == 0 && HALO % C == 0, "window edges split no half and no lane");
-    const bool cols = col >= own_c0 && col < own_c1;
-    const bool top = cols && row >= own_r0 && row < own_r1;
-    const bool bottom = cols && row + N >= own_r0 && row + N < own_r1;
-    const int n = own_c1 - col;
+    // ---- owned rows out
+    if (OUT_U) {
+        float *ub = P.u + (int64_t)frame * P.fs;
+        store(ub, u);
+        if (PROJ == 3 || (PROJ == 0 && !TAPE && P.resid)) {
+            f2 t[N][C];  // u - f, or t = u + (u - f)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        if (!(h ? bottom : top)) continue;
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            const int r = row + j + h * N;
-            if (EDGE && r >= H) break;
-            const unsigned o = (unsigned)r * (unsigned)W + col;
-            float a[C], b[C];
-            if (OUT_U) {
+            for (int j = 0; j < N; ++j)
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
-                    a[c] = h ? hi(u[j][c]) : lo(u[j][c]);
-                    b[c] = a[c] - (h ? hi(f[j][c]) : lo(f[j][c]));
+                    t[j][c] = sub2(u[j][c], f[j][c]);
+                    if (PROJ == 3) t[j][c] = add2(u[j][c], t[j][c]);
                 }
-                store_cols<C, MODE>(P.u + (int64_t)frame * P.fs + o, n, a);
-                if (PROJ == 3) {  // t = u + (u - f)
-#pragma unroll
-                    for (int c = 0; c < C; ++c) b[c] = a[c] + b[c];
-                    store_cols<C, MODE>(P.tout + (int64_t)frame * P.fs + o, n, b);
-                } else if (PROJ == 0 && P.resid) {
-                    store_cols<C, MODE>(P.resid + (int64_t)frame * P.fs + o, n, b);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    a[c] = h ? hi(pr[j][c]) : lo(pr[j][c]);
-                    b[c] = h ? hi(pc[j][c]) : lo(pc[j][c]);
-                }
-                float *pb = P.p_out + (int64_t)frame * 2 * hw + o;
-                store_cols<C, MODE>(pb, n, a);
-                store_cols<C, MODE>(pb + hw, n, b);
-            }
+            store((PROJ == 3 ? P.tout : P.resid) + (int64_t)frame * P.fs, t);
         }
+    } else if (!TAPE) {
+        float *pb = P.p_out + (int64_t)frame * 2 * hw;
+        store(pb, pr);
+        store(pb + hw, pc);
     }
 
     if (ENERGY) {
@@ -370,13 +443,14 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
     }
 }
 
-template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ>
+template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ, bool TAPE = false>
 __device__ __forceinline__ void run_mode(const Pass &P, int frame, int tr, int tc, int nup,
                                          Smem<C, NW> &sm) {
     const bool edge = tr == 0 || tr == P.nchunks - 1 || tc == 0 || tc == P.nbands - 1;
-    if (!P.vec) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, EDGE_SCALAR>(P, frame, tr, tc, nup, sm);
-    else if (edge) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, EDGE_VEC>(P, frame, tr, tc, nup, sm);
-    else run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, INSIDE>(P, frame, tr, tc, nup, sm);
+    if (TAPE && P.vec < 0) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, TAPE ? EDGE_WIDE : EDGE_SCALAR>(P, frame, tr, tc, nup, sm);
+    else if (!P.vec) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, EDGE_SCALAR>(P, frame, tr, tc, nup, sm);
+    else if (edge) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, EDGE_VEC>(P, frame, tr, tc, nup, sm);
+    else run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, INSIDE>(P, frame, tr, tc, nup, sm);
 }
 
 // Block -> (frame, window); the frames of a window are adjacent blocks (they
@@ -401,6 +475,18 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_tv_tile(Pass P) {
         __syncwarp();
         decide_stops(P, threadIdx.x);
     }
+}
+
+// A run of P.S updates of v = x + lam (q phi) that writes its tape, and u with
+// OUT_U; no stop test.
+template <int C, int N, int NW, int MINB, bool OUT_U>
+__global__ void __launch_bounds__(NW * 32, MINB) k_tv_tile_tape(Pass P) {
+    __shared__ Smem<C, NW> sm;
+    grid_dep_wait();
+    if (P.early) grid_dep_launch();
+    int frame, tr, tc;
+    decode(P, frame, tr, tc);
+    run_mode<C, N, NW, false, OUT_U, false, 2, true>(P, frame, tr, tc, P.S, sm);
 }
 
 // Frames whose rule fired at step j in this pass's window, with j - a updates.

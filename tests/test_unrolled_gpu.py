@@ -116,3 +116,16 @@ def test_unrolled_batch16_against_autograd():
     assert rel(g1, g2) < GRAD_REL
     assert rel(m1, m2) < GRAD_REL
     assert rel(g1, g3) < GRAD_REL
+
+
+# The tape / adjoint kernels' windows (64 x 32 pixels, 56 x 24 owned) and the
+# frames per launch, and the projection adjoint's item lanes (8, up to 4 items
+# at a time) and pixel groups (4, or 1 where H W is not a multiple of 4):
+# sizes around each.  Same bar as above.
+@pytest.mark.parametrize("N,B,H,W,K,T", [
+    (1, 1, 2, 3, 2, 5), (1, 2, 24, 56, 2, 5), (1, 2, 25, 57, 2, 4), (2, 1, 32, 64, 2, 5),
+    (1, 2, 33, 65, 2, 5), (1, 2, 29, 63, 2, 5), (2, 2, 81, 119, 2, 3), (1, 3, 80, 122, 2, 5),
+    (7, 6, 130, 260, 2, 5),                             # 31 frames per launch, then 11
+    (9, 2, 9, 12, 2, 5), (20, 3, 7, 9, 2, 5), (35, 9, 8, 12, 2, 5)])
+def test_unrolled_window_and_lane_edges(N, B, H, W, K, T):
+    test_unrolled_matches_fp64_autograd(N, B, H, W, K, T)

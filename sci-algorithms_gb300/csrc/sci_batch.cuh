@@ -33,8 +33,15 @@ struct Table {
     int qp_prefix[MAXI + 1];    // 128-pixel projection tasks of the work queue
     int tv_prefix[MAXI + 1];    // TV work items (one warp each) of the per-phase launches
     int tq_prefix[MAXI + 1];    // TV work items of the work queue (tvq geometry)
+    // The work queue's order (sci_batch_queue.cu): one period of n slots,
+    // entry 3 s + phase is the first task of that phase in slot s; slots by
+    // which a phase of an item's iteration lies behind its residual.
+    int order[3 * MAXI + 1];
+    int lag[3];
     Item it[MAXI];
 };
+
+enum { PH_PROJ = 0, PH_TV = 1, PH_FIX = 2 };  // phases of a work-queue iteration
 
 // Progress of one persistent launch (zeroed before it): the task counter,
 // the give-up flag of the bounded waits and per item the finished tasks of

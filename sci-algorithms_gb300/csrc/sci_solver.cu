@@ -21,10 +21,17 @@ int tv_launch_impl(const float *f, float *u, float *resid, int64_t nf, int64_t H
                    int64_t fs, float weight, float eps, int K, int *steps, double *energy_out,
                    void *workspace, size_t ws_bytes, cudaStream_t s, int force_R, int flags,
                    const uint32_t *proj_bits, const float *proj_c, float proj_lam);
-bool tv_proj_supported(int64_t nf, int64_t W, int K);
+bool tv_proj_supported(int64_t nf, int64_t W, int K, bool packed);
+bool tvx_proj_supported(int kind, int64_t nf, int64_t W, int iters, bool packed);
+int tv_launch_phi(const float *f, float *u, int64_t nf, int64_t H, int64_t W, int64_t fs,
+                  float weight, float eps, int K, int *steps, void *workspace, size_t ws_bytes,
+                  cudaStream_t s, int flags, const float *phi, const float *proj_c,
+                  float proj_lam);
 int tvx_launch(int kind, const float *f, float *u, float *resid, int64_t nf, int64_t H,
                int64_t W, float lam, int iters, int *steps, void *ws, size_t ws_bytes,
-               cudaStream_t s);
+               cudaStream_t s, const uint32_t *proj_bits = nullptr,
+               const float *proj_phi = nullptr, const float *proj_c = nullptr,
+               float proj_lam = 0.f);
 size_t tvx_workspace_bytes(int kind, int64_t nf, int64_t H, int64_t W, int iters);
 int launch_proj_admm_tma(const float *th, const float *bb, const uint32_t *bits, const float *y,
                          const float *phisum, float *v, float *xo, float lam, float gamma, int B,
@@ -172,10 +179,14 @@ int enqueue(const Args &a, cudaStream_t s) {
     auto rn = [&](int it) { return o.resid_norm ? o.resid_norm + it : nullptr; };
     const bool aligned = ((reinterpret_cast<uintptr_t>(a.x0) | reinterpret_cast<uintptr_t>(a.x_out) |
                            reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.phisum) |
-                           reinterpret_cast<uintptr_t>(a.bits)) & 15u) == 0;
-    if (!a.admm && !o.tvm && a.bits && aligned && hw % 4 == 0 && tv_proj_supported(B, W, K)) {
+                           reinterpret_cast<uintptr_t>(a.bits) | (a.bits ? 0 : reinterpret_cast<uintptr_t>(a.phi))) & 15u) == 0;
+    const bool packed = a.bits != nullptr;
+    if (!a.admm && aligned && hw % 4 == 0 &&
+        (o.tvm ? tvx_proj_supported(o.tvm, B, W, K, packed) : tv_proj_supported(B, W, K, packed))) {
         // Fused iteration: a read-only pass forms the residual map c (and
         // y1); the TV kernel applies x + lambda (c phi_b) while it loads x.
+        // (With a float mask it reads phi once more, but writes and reads no
+        // projected stack.)
         // x ping-pongs between x_out and xp; start so the last iterate
         // lands in x_out.
         float *X[2] = {a.x_out, w.xp};
@@ -186,16 +197,25 @@ int enqueue(const Args &a, cudaStream_t s) {
         // the residual pass also clears the TV pass's stop-test sums, so
         // that the TV kernel follows it directly (flags 4)
         int nzero = 0;
-        double *zero = tv_clear_region(B, H, W, K, w.tv, &nzero);
+        double *zero = o.tvm ? nullptr : tv_clear_region(B, H, W, K, w.tv, &nzero);
+        const float *phi = packed ? nullptr : a.phi;
         for (int it = 0; it < o.iters; ++it) {
             const float *cur = X[(start + it) & 1];
             float *nxt = X[(start + it + 1) & 1];
-            int e = gap_residual_rn(cur, nullptr, a.bits, a.y, w.y1, a.phisum, w.c,
-                                    o.accelerate, B, H, W, s, rn(it), zero, nzero);
+            int *steps = o.tv_steps ? o.tv_steps + (int64_t)it * B : nullptr;
+            int e = gap_residual_rn(cur, phi, a.bits, a.y, w.y1, a.phisum, w.c, o.accelerate, B,
+                                    H, W, s, rn(it), zero, nzero);
             if (e) return e;
-            e = tv_launch_impl(cur, nxt, nullptr, B, H, W, hw, o.weights[it], o.eps, K,
-                               o.tv_steps ? o.tv_steps + (int64_t)it * B : nullptr, nullptr, w.tv,
-                               w.tv_bytes, s, 0, 4, a.bits, w.c, o.lambdas[it]);
+            if (o.tvm)  // the clip files take tvweight itself
+                e = tvx_launch(o.tvm, cur, nxt, nullptr, B, H, W, o.weights[it], K, steps, w.tv,
+                               w.tv_bytes, s, a.bits, phi, w.c, o.lambdas[it]);
+            else if (!packed)
+                e = tv_launch_phi(cur, nxt, B, H, W, hw, o.weights[it], o.eps, K, steps, w.tv,
+                                  w.tv_bytes, s, 4, phi, w.c, o.lambdas[it]);
+            else
+                e = tv_launch_impl(cur, nxt, nullptr, B, H, W, hw, o.weights[it], o.eps, K, steps,
+                                   nullptr, w.tv, w.tv_bytes, s, 0, 4, a.bits, w.c,
+                                   o.lambdas[it]);
             if (e) return e;
             if (o.orig && o.sqerr) {
                 e = sci_sqerr_accum(o.orig, nxt, n, o.sqerr + it, s);
@@ -225,7 +245,7 @@ int enqueue(const Args &a, cudaStream_t s) {
     // admm_denoise: theta = x0, b = 0  (pnp_sci_algo.py:800-802)
     SCI_CUDA(cudaMemcpyAsync(w.theta, a.x0, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
     const char *af = getenv("SCI_ADMM_FUSED");
-    if (!o.tvm && a.bits && aligned && hw % 4 == 0 && tv_proj_supported(B, W, K) &&
+    if (!o.tvm && a.bits && aligned && hw % 4 == 0 && tv_proj_supported(B, W, K, true) &&
         !(af && af[0] == '0')) {
         // Fused iteration: a read-only pass forms the residual map r_k from
         // t_k = theta_k + b_k; the TV kernel applies theta_k + lambda_k

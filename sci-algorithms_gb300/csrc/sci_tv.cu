@@ -224,6 +224,9 @@ struct RuleArgs {
     // with the on-load projection: also store t = u + (u - f) (the lean
     // pass only, PROJ 3; the fused ADMM iteration's next t = theta + b)
     float *tout = nullptr;
+    // the on-load projection's mask as floats, one plane per frame, instead of
+    // packed (the lean pass and the tiles)
+    const float *phi = nullptr;
 };
 
 static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, int64_t H,
@@ -232,19 +235,21 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
                           int force_R, int flags, const uint32_t *proj_bits, const float *proj_c,
                           float proj_lam, const RuleArgs &ra) {
     const bool no_stop = (flags & 1) != 0 || ra.rule != tv::RULE_SKIMAGE;
-    const bool proj = proj_bits != nullptr;
+    const bool proj = proj_bits != nullptr || ra.phi != nullptr;
     using namespace tv;
     SCI_CHECK_ARG(f && u && nf >= 1 && H >= 1 && W >= 1, "tv: bad arguments");
     SCI_CHECK_ARG(K >= 1, "tv: n_iter_max must be >= 1");
     SCI_CHECK_ARG(weight > 0.f, "tv: weight must be > 0 (got %g)", (double)weight);
-    SCI_CHECK_ARG(!proj || ra.rule == RULE_SKIMAGE, "tv: on-load projection needs the default rule");
+    SCI_CHECK_ARG(!proj || ra.rule == RULE_SKIMAGE || ra.rule == RULE_CLIP,
+                  "tv: on-load projection needs the default or the clip rule");
     SCI_CHECK_ARG(f != u, "tv: input and output must not alias");
     SCI_CHECK_ARG(H <= (1 << 30) && W <= (1 << 30) && nf <= (1 << 30), "tv: sizes too large");
     const size_t need = ws_layout(nf, H, W, K, nullptr, nullptr);
     SCI_CHECK_ARG(workspace && ws_bytes >= need, "tv: workspace of %zu bytes needed, got %zu",
                   need, ws_bytes);
     if (proj) {
-        SCI_CHECK_ARG(proj_c && nf <= 32 && K >= 2 && K <= SMAX + 1 && !resid && !no_stop,
+        SCI_CHECK_ARG(proj_c && (ra.phi || nf <= 32) && K >= 2 && K <= SMAX + 1 && !resid &&
+                          (!no_stop || ra.rule == RULE_CLIP),
                       "tv: on-load projection needs K in [2, 5], nf <= 32, no resid");
     }
     if (K == 1) {
@@ -287,7 +292,8 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
         return (W % c == 0) && (fs % c == 0) && W >= c &&
                ((reinterpret_cast<uintptr_t>(f) | reinterpret_cast<uintptr_t>(u) |
                  reinterpret_cast<uintptr_t>(resid) | reinterpret_cast<uintptr_t>(proj_bits) |
-                 reinterpret_cast<uintptr_t>(proj_c)) % (4 * c) == 0);
+                 reinterpret_cast<uintptr_t>(proj_c) | reinterpret_cast<uintptr_t>(ra.phi)) %
+                    (4 * c) == 0);
     };
     // flags bits 8-11: columns per lane forced by the caller (2 or 4)
     const int fcpl = (flags >> 8) & 0xf;
@@ -296,7 +302,12 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
                       (!ra.tout || (reinterpret_cast<uintptr_t>(ra.tout) % (4 * cpl_pick)) == 0);
     SCI_CHECK_ARG(!ra.tout || (proj && slim), "tv: the t output needs the lean pass with the "
                                               "on-load projection (aligned frames)");
-    const int pmode = proj ? (ra.tout ? 3 : 1) : 0;  // the lean pass's PROJ
+    const int pmode = proj ? (ra.tout ? 3 : (ra.phi ? 2 : 1)) : 0;  // the lean pass's PROJ
+    // the clip rule in one pass on the lean pipeline (4 columns per lane)
+    const bool clip = slim_enabled() && ra.rule == RULE_CLIP && !resid && U <= SMAX &&
+                      force_R <= 0 && !getenv("SCI_TV_R") && aligned_for(4);
+    SCI_CHECK_ARG(!proj || slim || clip || !(ra.phi || ra.rule == RULE_CLIP),
+                  "tv: this on-load projection needs the lean pass (aligned frames)");
     const int cpl = slim ? cpl_pick : ((proj || ra.rule != RULE_SKIMAGE) ? 4 : cpl_pick);
     const bool vec = (W % cpl == 0) && (fs % cpl == 0) &&
                      ((reinterpret_cast<uintptr_t>(f) | reinterpret_cast<uintptr_t>(u) |
@@ -347,13 +358,15 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
         P.tout = ra.tout;
         P.bits = proj_bits;
         P.cmap = proj_c;
+        P.phi = ra.phi;
         P.lam = proj_lam;
         P.frame_fast = frame_fast_order(proj);
         P.nbands = band_count((int)W, 32 * cpl, P.hl, P.hr);
         if (force_R > 0) P.R = force_R;
-        else if (slim)
+        else if (slim || clip)
             P.R = choose_R_slim(nf, P.nbands, (int)H, SG,
-                                kSMs * slim_resident_blocks(cpl, SG, minb, pmode));
+                                kSMs * (clip ? clip_resident_blocks()
+                                             : slim_resident_blocks(cpl, SG, minb, pmode)));
         else P.R = choose_R(nf, P.nbands, (int)H);
         P.nchunks = (int)((H + P.R - 1) / P.R);
         P.S = SG;
@@ -372,6 +385,9 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
             tile_geometry(P);
             P.early = tile_blocks(P) > kSMs * tile_resident_blocks();
             launch_tile(P, PIN, FINAL, pmode, s);
+        } else if (clip) {
+            P.early = pass_blocks(P) > (unsigned)(kSMs * clip_resident_blocks());
+            launch_clip(P, SG, pmode, s);
         } else if (slim) {
             P.early = pass_blocks(P) > (unsigned)(kSMs * slim_resident_blocks(cpl, SG, minb, pmode));
             launch_slim(P, SG, minb, pmode, s);
@@ -413,6 +429,17 @@ int tv_launch_impl(const float *f, float *u, float *resid, int64_t nf, int64_t H
                           RuleArgs{});
 }
 
+// tv_launch_impl with the on-load projection of a float mask.
+int tv_launch_phi(const float *f, float *u, int64_t nf, int64_t H, int64_t W, int64_t fs,
+                  float weight, float eps, int K, int *steps, void *workspace, size_t ws_bytes,
+                  cudaStream_t s, int flags, const float *phi, const float *proj_c,
+                  float proj_lam) {
+    RuleArgs ra;
+    ra.phi = phi;
+    return tv_launch_core(f, u, nullptr, nf, H, W, fs, weight, eps, K, steps, nullptr, workspace,
+                          ws_bytes, s, 0, flags, nullptr, proj_c, proj_lam, ra);
+}
+
 // tv_launch_impl with the on-load projection that also stores t = u + (u -
 // f) into tout (the lean pass; see RuleArgs::tout).
 int tv_launch_tout(const float *f, float *u, int64_t nf, int64_t H, int64_t W, int64_t fs,
@@ -429,7 +456,8 @@ int tv_launch_tout(const float *f, float *u, int64_t nf, int64_t H, int64_t W, i
 // sci_tv.cuh); the workspace is tv_workspace_bytes(nf, H, W, updates + 1).
 int tv_launch_rule(int rule, const float *f, float *u, float *resid, int64_t nf, int64_t H,
                    int64_t W, int updates, float tau, float tw, float c1, float c2, int *steps,
-                   void *workspace, size_t ws_bytes, cudaStream_t s) {
+                   void *workspace, size_t ws_bytes, cudaStream_t s, const uint32_t *proj_bits,
+                   const float *proj_phi, const float *proj_c, float proj_lam) {
     SCI_CHECK_ARG(rule >= tv::RULE_CHAM_ITV && rule <= tv::RULE_CLIP && updates >= 0,
                   "tv: bad rule arguments");
     RuleArgs ra;
@@ -438,8 +466,9 @@ int tv_launch_rule(int rule, const float *f, float *u, float *resid, int64_t nf,
     ra.tw = tw;
     ra.c1 = c1;
     ra.c2 = c2;
+    ra.phi = proj_phi;
     return tv_launch_core(f, u, resid, nf, H, W, H * W, 1.0f, 0.f, updates + 1, steps, nullptr,
-                          workspace, ws_bytes, s, 0, 1, nullptr, nullptr, 0.f, ra);
+                          workspace, ws_bytes, s, 0, 1, proj_bits, proj_c, proj_lam, ra);
 }
 
 int tv_launch_flags(const float *f, float *u, float *resid, int64_t nf, int64_t H, int64_t W,
@@ -456,17 +485,20 @@ int tv_launch(const float *f, float *u, float *resid, int64_t nf, int64_t H, int
                            workspace, ws_bytes, s, force_R, 0);
 }
 
-// The on-load projection path covers one measurement of <= 32 frames with a
-// packed mask, 2..5 Chambolle steps (one pass) and 16-byte aligned rows.
+// The on-load projection path covers one measurement with a packed (<= 32
+// frames) or float mask, 2..5 Chambolle steps (one pass) and 16-byte aligned rows.
 // On by default (SCI_FUSED_PROJ=0 turns it off): with the lean TV pass,
 // whose input rows come through shared-memory rings, the projection costs
 // the pass little, and the iteration at 2048 x 2048 x 24 goes from 2123 to
 // 2180-2187 iter/s (residual pass 73 us instead of the 141 us projection).
 // With the generic pipeline it was slower (552 + 73 us against 385 + 179).
-bool tv_proj_supported(int64_t nf, int64_t W, int K) {
+// packed: the mask is packed (nf <= 32 bits of a word); the clip rule takes
+// its updates + 1 as K.
+bool tv_proj_supported(int64_t nf, int64_t W, int K, bool packed) {
     const char *e = getenv("SCI_FUSED_PROJ");
-    return !(e && atoi(e) == 0) && slim_enabled() && nf <= 32 && K >= 2 &&
-           K <= tv::SMAX + 1 && W % 4 == 0 && !getenv("SCI_TV_LAG");
+    return !(e && atoi(e) == 0) && slim_enabled() && (!packed || nf <= 32) && K >= 2 &&
+           K <= tv::SMAX + 1 && W % 4 == 0 && !getenv("SCI_TV_LAG") &&
+           (packed || !getenv("SCI_SLIM_MINB"));
 }
 
 size_t tv_workspace_bytes(int64_t nf, int64_t H, int64_t W, int K) {

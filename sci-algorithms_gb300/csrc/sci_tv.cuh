@@ -105,8 +105,9 @@ struct Pass {
     // t = u + (u - f) of every frame, same layout as u (nullable otherwise).
     float *tout;
     int early;            // more blocks than fit at once: grid_dep_launch()
-    // Unrolled solver (sci_tv_tile.cuh, PROJ 2): frames are frames frame0 ..
-    // of N scenes of B; f holds x, cmap the scenes' maps q, phi [B][H][W].
+    // phi: a float mask, one plane per frame (the lean pass's PROJ 2, tiles'
+    // 4).  Unrolled solver (tiles' PROJ 2): frames are frames frame0 .. of N
+    // scenes of B; f holds x, cmap the scenes' maps q, phi [B][H][W].
     const float *phi, *lam_dev;
     int frame0, B;
 };
@@ -940,6 +941,8 @@ bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim);  // sci_tv_tile.cu
 void tile_geometry(Pass &P);
 int tile_columns();
 int64_t tile_blocks(const Pass &P);
+void launch_clip(const Pass &P, int SG, int proj, cudaStream_t s);  // sci_tv_clip.cu
+int clip_resident_blocks();
 int tile_resident_blocks();
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s);
 void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s);

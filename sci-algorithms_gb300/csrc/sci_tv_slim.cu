@@ -11,8 +11,8 @@ void launch_slim2(const Pass &P, int SG, int minb, int proj, cudaStream_t s);  /
 void launch_slim2_fix(const Pass &P, int proj, cudaStream_t s);
 int slim2_resident_blocks(int SG, int minb, int proj);
 
-// proj: 0 none, 1 the GAP projection on load, 3 also the t output (the
-// default register budget only)
+// proj: 0 none, 1 the GAP projection on load, 2 with a float mask, 3 (packed
+// mask) also the t output (2, 3: the default register budget only)
 void launch_slim(const Pass &P, int SG, int minb, int proj, cudaStream_t s) {
     using namespace slim;
     if (P.cpl == 2) return launch_slim2(P, SG, minb, proj, s);
@@ -23,6 +23,8 @@ void launch_slim(const Pass &P, int SG, int minb, int proj, cudaStream_t s) {
     const int form = (e && atoi(e) == 0) ? 0 : 1;
     if (proj == 3) {
         launch_main<4, 4, 3>(P, SG, s, form);
+    } else if (proj == 2) {
+        launch_main<4, 4, 2>(P, SG, s);
     } else if (minb == 3) {
         if (proj) launch_main<4, 3, 1>(P, SG, s);
         else launch_main<4, 3, 0>(P, SG, s);
@@ -37,6 +39,7 @@ void launch_slim_fix(const Pass &P, int proj, cudaStream_t s) {
     if (P.cpl == 2) return launch_slim2_fix(P, proj, s);
     constexpr int D = MinB<4>::def;
     if (proj == 3) (void)launch_dep(k_tv_slim_fix<4, D, 3>, dim3(pass_blocks(P)), dim3(WPB * 32), 0, s, P);
+    else if (proj == 2) (void)launch_dep(k_tv_slim_fix<4, D, 2>, dim3(pass_blocks(P)), dim3(WPB * 32), 0, s, P);
     else if (proj) (void)launch_dep(k_tv_slim_fix<4, D, 1>, dim3(pass_blocks(P)), dim3(WPB * 32), 0, s, P);
     else (void)launch_dep(k_tv_slim_fix<4, D, 0>, dim3(pass_blocks(P)), dim3(WPB * 32), 0, s, P);
 }
@@ -47,11 +50,12 @@ int slim_resident_blocks(int cpl, int SG, int minb, int proj) {
     static std::mutex mu;
     static int cache[2][4][5] = {};
     SG = SG < 1 ? 1 : (SG > 4 ? 4 : SG);
-    const int mi = (minb == 3 && proj != 3) ? 0 : 1;
+    const int mi = (minb == 3 && proj < 2) ? 0 : 1;
     std::lock_guard<std::mutex> lock(mu);
     int &v = cache[mi][proj & 3][SG];
     if (v == 0) {
         const void *k = proj == 3 ? main_kernel<4, 4, 3>(SG)
+                        : proj == 2 ? main_kernel<4, 4, 2>(SG)
                         : mi == 0 ? (proj ? main_kernel<4, 3, 1>(SG) : main_kernel<4, 3, 0>(SG))
                                   : (proj ? main_kernel<4, 4, 1>(SG) : main_kernel<4, 4, 0>(SG));
         v = resident(k, mi == 0 ? 3 : 4);

@@ -26,7 +26,11 @@
 // input ring for the later stages.  PROJ 3 is PROJ 1 that also stores
 // t = u + (u - f) beside u (P.tout): in the ADMM iteration f is the TV
 // input v = x - b and u the new theta, so t = theta + b of the next
-// projection.
+// projection.  PROJ 2 is PROJ 1 with a float mask (P.phi, one plane per frame):
+// f = x + lam (c phi_b).
+//
+// The MATLAB clip files (RULE_CLIP of sci_tv.cuh) run on the same pipeline as
+// FORM 2: no norm, no MUFU, no energies.
 //
 // Rounding is identical to the generic pipeline (same operations in the same
 // order), so the two produce bit-identical frames.
@@ -145,7 +149,7 @@ struct Rings {
 // (ldb: the pair's bytes inside the frame) and sstep synchronises the warp.
 template <int CPL, int PROJ, int COH = 0>
 __device__ __forceinline__ void fetch(const Pass &P, const Rings &G, const float *fb, int slot,
-                                      int row, int colc, uint32_t ldb) {
+                                      int row, int colc, uint32_t ldb, int frame) {
     const int64_t o = (int64_t)row * P.W + colc;
     const uint32_t so = (uint32_t)(slot & (RING - 1)) * Geo<CPL>::ROWB;
     if (COH && CPL == 2) {
@@ -160,7 +164,10 @@ __device__ __forceinline__ void fetch(const Pass &P, const Rings &G, const float
         cp_row<CPL>(G.xs + so, fb + o, ldb);
         if (PROJ) {
             cp_row<CPL>(G.cs + so, P.cmap + o, ldb);
-            cp_row<CPL>(G.ms + so, P.bits + o, ldb);
+            if (PROJ == 2)
+                cp_row<CPL>(G.ms + so, P.phi + (int64_t)frame * P.H * P.W + o, ldb);
+            else
+                cp_row<CPL>(G.ms + so, P.bits + o, ldb);
         }
     }
     cp_commit();
@@ -178,7 +185,8 @@ __device__ __forceinline__ Row<CPL> stage0(const Pass &P, const Rings &G, int r,
         const uint32_t fbit = 1u << frame;
 #pragma unroll
         for (int j = 0; j < NQ; ++j)
-            u.q[j] = mk2(proj_px(P.lam, lo(c.q[j]), lo(u.q[j]), __float_as_uint(lo(wb.q[j])), fbit),
+            if (PROJ == 2) u.q[j] = fma2(mk2(P.lam, P.lam), mul2(c.q[j], wb.q[j]), u.q[j]);
+            else u.q[j] = mk2(proj_px(P.lam, lo(c.q[j]), lo(u.q[j]), __float_as_uint(lo(wb.q[j])), fbit),
                          proj_px(P.lam, hi(c.q[j]), hi(u.q[j]), __float_as_uint(hi(wb.q[j])), fbit));
         sts<CPL>(G.x, r, u);
     }
@@ -203,7 +211,7 @@ __device__ __forceinline__ void stage(const Pass &P, const SS<S, CPL> &in, SS<S,
     constexpr int NQ = Geo<CPL>::NQ;
     const int H = P.H, W = P.W;
     const f2 one2 = mk2(1.f, 1.f), tw2 = mk2(P.tw, P.tw);
-    const f2 nt2 = FORM ? mk2(-0.25f, -0.25f) : mk2(-P.tau, -P.tau);
+    const f2 nt2 = FORM == 1 ? mk2(-0.25f, -0.25f) : mk2(-P.tau, -P.tau);
     const f2 w2 = FORM ? mk2(16.f * P.weight, 16.f * P.weight) : mk2(P.weight, P.weight);
     const int i = r - K;
     out.up[K - 1] = ucur;  // u_{K-1}(i+1): stage K's row in the next step
@@ -225,6 +233,15 @@ __device__ __forceinline__ void stage(const Pass &P, const SS<S, CPL> &in, SS<S,
         gc.q[j] = mk2(hi(up.q[j]) - lo(up.q[j]), nx - hi(up.q[j]));
         if (MODE != INTERIOR) gc.q[j] = mul2(gc.q[j], L.gmask.q[j]);
         gr.q[j] = (GEN && i == H - 1) ? mk2(0.f, 0.f) : sub2(ucur.q[j], up.q[j]);
+        if constexpr (FORM == 2) {  // clamp(p - tau g, -c1, c1)
+            const f2 zero = mk2(0.f, 0.f);
+            const f2 tr = fma2(nt2, gr.q[j], K == 1 ? zero : in.pr[K - 1].q[j]);
+            const f2 tc = fma2(nt2, gc.q[j], K == 1 ? zero : in.pc[K == 1 ? 0 : K - 1].q[j]);
+            const float c = P.c1;
+            prn.q[j] = mk2(fminf(fmaxf(lo(tr), -c), c), fminf(fmaxf(hi(tr), -c), c));
+            pcn.q[j] = mk2(fminf(fmaxf(lo(tc), -c), c), fminf(fmaxf(hi(tc), -c), c));
+            continue;
+        }
         const f2 s = fma2(gr.q[j], gr.q[j], mul2(gc.q[j], gc.q[j]));
         n.q[j] = mk2(sqrt_approx(lo(s)), sqrt_approx(hi(s)));
         const f2 den = fma2(tw2, n.q[j], one2);
@@ -253,7 +270,9 @@ __device__ __forceinline__ void stage(const Pass &P, const SS<S, CPL> &in, SS<S,
         const f2 t = sub2(add2(prn.q[j], pcn.q[j]), in.pr[K].q[j]);
         const float left = (j == 0) ? pcl : hi(pcn.q[(j + NQ - 1) % NQ]);
         d.q[j] = mk2(lo(t) - left, hi(t) - lo(pcn.q[j]));
-        uk.q[j] = FORM ? fma2(nt2, d.q[j], fi.q[j]) : sub2(fi.q[j], d.q[j]);
+        uk.q[j] = FORM == 2   ? fma2(mk2(-P.c2, -P.c2), d.q[j], fi.q[j])
+                  : FORM == 1 ? fma2(nt2, d.q[j], fi.q[j])
+                              : sub2(fi.q[j], d.q[j]);
     }
     out.pr[K] = prn;
     if (K < S) out.pc[K] = pcn;
@@ -303,7 +322,7 @@ __device__ __forceinline__ void sstep(const Pass &P, const SS<S, CPL> &in, SS<S,
                                       int frame, f2 (&ek)[S]) {
     // copy input row r + PF into its ring slots (clamped into the frame; a
     // clamped row is never read), then wait for row r
-    fetch<CPL, PROJ, COH>(P, G, fb, r + PF, min(r + PF, P.H - 1), L.colc, ldb);
+    fetch<CPL, PROJ, COH>(P, G, fb, r + PF, min(r + PF, P.H - 1), L.colc, ldb, frame);
     cp_wait<PF>();
     if (COH && CPL == 2) __syncwarp();  // the pair's copy was the even lane's
     Row<CPL> ucur = (!GEN || r < P.H) ? stage0<CPL, PROJ>(P, G, r, frame) : zrow<CPL>();
@@ -347,7 +366,7 @@ __device__ __forceinline__ void srun(const Pass &P, int frame, int chunk, int ba
     // the first PF input rows
 #pragma unroll
     for (int q = 0; q < PF; ++q)
-        fetch<CPL, PROJ, COH>(P, G, fb, rs + q, min(rs + q, H - 1), L.colc, ldb);
+        fetch<CPL, PROJ, COH>(P, G, fb, rs + q, min(rs + q, H - 1), L.colc, ldb, frame);
 
     SS<S, CPL> A, B;
     zero_ss<S, CPL>(A);
@@ -443,6 +462,18 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_tv_slim(Pass P) {
     srun_mode<S, CPL, true, PROJ, FORM>(P, frame, chunk, band, lane,
                                         lane_rings<CPL, PROJ>(smem, lane));
     if (P.ticket) decide_stops(P, lane);
+}
+
+// A single-pass run of the clip rule: S updates of every frame, no stop test.
+template <int S, int MINB, int PROJ>
+__global__ void __launch_bounds__(WPB * 32, MINB) k_tv_slim_clip(Pass P) {
+    __shared__ __align__(16) unsigned char smem[Smem<4, PROJ>::bytes];
+    grid_dep_wait();
+    if (P.early) grid_dep_launch();
+    int frame, chunk, band;
+    if (!decode_item(P, frame, chunk, band)) return;
+    const int lane = threadIdx.x & 31;
+    srun_mode<S, 4, false, PROJ, 2>(P, frame, chunk, band, lane, lane_rings<4, PROJ>(smem, lane));
 }
 
 // Stop-test launch of a single-pass run: frames whose rule fired at step j

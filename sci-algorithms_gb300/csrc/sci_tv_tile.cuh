@@ -176,7 +176,7 @@ struct Cells {
 
 // One row of the input f of a frame (its stack at fb): the stored values, or
 // with the projection applied as it is loaded -- PROJ 1, 3: a packed binary
-// mask (proj_px); PROJ 2: the unrolled solver's v = x + lam (q phi_b), with a
+// mask (proj_px); PROJ 4: a float mask; PROJ 2: the unrolled solver's v = x + lam (q phi_b), with a
 // float mask per frame of a scene, the map q per scene and lam in device
 // memory.
 template <int PROJ, int C, int N, int MODE, typename Args>
@@ -192,6 +192,12 @@ __device__ __forceinline__ void load_f(const Args &P, const Cells<C, N, MODE> &X
 #pragma unroll
         for (int c = 0; c < C; ++c)
             v[c] = proj_px(P.lam, cm[c], v[c], __float_as_uint(wb[c]), 1u << frame);
+    } else if constexpr (PROJ == 4) {
+        float q[C], m[C];
+        X.load(P.cmap, o, in, q);
+        X.load(P.phi + (int64_t)frame * P.H * P.W, o, in, m);
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = fmaf(P.lam, q[c] * m[c], v[c]);
     } else if constexpr (PROJ == 2) {
         const int64_t hw = (int64_t)P.H * P.W;
         const int g = P.frame0 + frame, n = g / P.B;

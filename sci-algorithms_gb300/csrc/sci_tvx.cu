@@ -39,8 +39,11 @@ namespace sci {
 
 int tv_launch_rule(int rule, const float *f, float *u, float *resid, int64_t nf, int64_t H,
                    int64_t W, int updates, float tau, float tw, float c1, float c2, int *steps,
-                   void *workspace, size_t ws_bytes, cudaStream_t s);
+                   void *workspace, size_t ws_bytes, cudaStream_t s,
+                   const uint32_t *proj_bits = nullptr, const float *proj_phi = nullptr,
+                   const float *proj_c = nullptr, float proj_lam = 0.f);
 size_t tv_workspace_bytes(int64_t nf, int64_t H, int64_t W, int K);
+bool tv_proj_supported(int64_t nf, int64_t W, int K, bool packed);
 
 namespace tvx {
 
@@ -468,11 +471,20 @@ size_t tvx_workspace_bytes(int kind, int64_t nf, int64_t H, int64_t W, int iters
     return sizeof(float) * (size_t)planes * (size_t)(nf * H * W);
 }
 
+// The on-load projection covers the clip kinds in one pass.
+bool tvx_proj_supported(int kind, int64_t nf, int64_t W, int iters, bool packed) {
+    return (kind == tvx::CLIP_A || kind == tvx::CLIP_B) &&
+           tv_proj_supported(nf, W, iters, packed);
+}
+
 // kind 1..8 as above; lambda and iters are the denoiser's own parameters
 // (gapdenoise.m passes tvweight or 1/tvweight, and 5 or 2 iterations).
+// proj_c (nullable, tvx_proj_supported): the GAP projection f = x + proj_lam
+// (proj_c phi_b) applied as the input is loaded, with a packed or float mask.
 int tvx_launch(int kind, const float *f, float *u, float *resid, int64_t nf, int64_t H,
                int64_t W, float lam, int iters, int *steps, void *ws, size_t ws_bytes,
-               cudaStream_t s) {
+               cudaStream_t s, const uint32_t *proj_bits, const float *proj_phi,
+               const float *proj_c, float proj_lam) {
     using namespace tvx;
     SCI_CHECK_ARG(kind >= CLIP_A && kind <= FGP_ITV3D, "tv_matlab: unknown kind %d", kind);
     SCI_CHECK_ARG(f && u && f != u && nf >= 1 && H >= 2 && W >= 2 && iters >= 1,
@@ -507,7 +519,8 @@ int tvx_launch(int kind, const float *f, float *u, float *resid, int64_t nf, int
             // last iteration sees iters-1 dual updates; 1/alpha = 1/5
             return tv_launch_rule(tv::RULE_CLIP, f, u, resid, nf, H, W, iters - 1, 0.2f, 0.f,
                                   kind == CLIP_A ? lam / 2 : lam, kind == CLIP_A ? 0.5f : 1.f,
-                                  nullptr, ws, ws_bytes, s);
+                                  nullptr, ws, ws_bytes, s, proj_bits, proj_phi, proj_c,
+                                  proj_lam);
         case CHAM_ITV2D:
             // tvdenoise_cham_ITV2D.m:62-93: every iteration's update is live
             return tv_launch_rule(tv::RULE_CHAM_ITV, f, u, resid, nf, H, W, iters, 0.125f,
@@ -585,7 +598,8 @@ int sci_tv_matlab(int kind, const float *f, float *u, int64_t nframes, int64_t H
                   float lambda, int iters, void *workspace, size_t workspace_bytes,
                   void *stream) {
     return sci::tvx_launch(kind, f, u, nullptr, nframes, H, W, lambda, iters, nullptr, workspace,
-                           workspace_bytes, sci::as_stream(stream));
+                           workspace_bytes, sci::as_stream(stream), nullptr, nullptr, nullptr,
+                           0.f);
 }
 
 }  // extern "C"

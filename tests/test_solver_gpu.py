@@ -313,3 +313,48 @@ def test_fused_admm_iteration(monkeypatch, shape, cpl, with_orig):
     assert np.allclose(ra, rb, rtol=1e-4, atol=0)
     if with_orig:
         assert np.allclose(pa, pb, rtol=0, atol=1e-3)
+
+
+# The fused iteration with a float mask (the lean pass's and the tiles'
+# projection on load) and with the clip denoisers (their lean pass, packed and
+# float masks) against the projection kernel and the plain denoiser: the same
+# operations, so the same bits.  Widths around the 128-column bands and the
+# 64-column windows, 1 to 4 updates, more than 32 float-masked frames.
+@pytest.mark.parametrize("H,W,B", [(2, 4, 1), (7, 128, 3), (33, 132, 2), (50, 248, 4),
+                                   (97, 252, 5), (48, 64, 33), (130, 1028, 2)])
+@pytest.mark.parametrize("gray", [True, False])
+@pytest.mark.parametrize("tvm,K", [("tv_chambolle", 2), ("tv_chambolle", 5), ("ATV_ClipA", 5),
+                                   ("ATV_ClipB", 5)])
+def test_fused_float_mask_and_clip_are_bitwise_equal(monkeypatch, H, W, B, gray, tvm, K):
+    if not gray and B > 32:
+        pytest.skip("a packed mask holds 32 frames")
+    g = torch.Generator(device="cuda").manual_seed(H * W + B)
+    mask = torch.rand(H, W, B, device="cuda", generator=g)
+    if not gray:
+        mask = (mask < 0.5).float()
+    op = sci.MaskOperator(mask)
+    assert (op.bits is None) == gray
+    y = op.phi.sum(0) * torch.rand(H, W, device="cuda", generator=g)
+    for acc in (True, False):
+        out = []
+        for fused, tile in (("0", "0"), ("1", "0"), ("1", "1")):
+            monkeypatch.setenv("SCI_FUSED_PROJ", fused)
+            monkeypatch.setenv("SCI_TV_TILE", tile)
+            s = sci.Solver(op, "gap", 5, 0.9, 0.1, K, tvm=tvm, accelerate=acc, eps=0.02,
+                           use_graph=False)
+            out.append((s.run(y, tv_steps=True).clone(), s.tv_steps.clone()))
+        for x, steps in out[1:]:
+            assert torch.equal(out[0][0], x)
+            assert torch.equal(out[0][1], steps)
+
+
+@pytest.mark.parametrize("H,W,F", [(2, 4, 2), (9, 128, 1), (40, 132, 3), (100, 520, 2)])
+@pytest.mark.parametrize("iters", [2, 3, 4, 5, 7])
+@pytest.mark.parametrize("tvm", ["ATV_ClipA", "ATV_ClipB"])
+def test_clip_lean_pass_is_bitwise_equal(monkeypatch, H, W, F, iters, tvm):
+    f = torch.rand(F, H, W, device="cuda", generator=torch.Generator("cuda").manual_seed(H + W))
+    out = []
+    for slim in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_SLIM", slim)
+        out.append(sci.tv_matlab_frames(f, tvm, 0.07, iters))
+    assert torch.equal(*out)

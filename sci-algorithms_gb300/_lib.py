@@ -121,6 +121,7 @@ _SIGS = {
 }
 
 _lib = None
+_fns = {}  # name -> bound function, once the library is loaded
 
 
 def lib_path():
@@ -142,6 +143,7 @@ def load(build_if_missing=True):
         fn = getattr(L, name)
         fn.argtypes = argt
         fn.restype = ctypes.c_int
+        _fns[name] = fn
     _lib = L
     return L
 
@@ -159,8 +161,10 @@ def last_error():
 
 def call(name, *args):
     """Call ``name`` and raise SciError on a negative status."""
-    L = load()
-    rc = getattr(L, name)(*args)
+    fn = _fns.get(name)
+    if fn is None:
+        fn = getattr(load(), name)
+    rc = fn(*args)
     if rc != SCI_OK:
         raise SciError(name, rc, last_error())
     return rc

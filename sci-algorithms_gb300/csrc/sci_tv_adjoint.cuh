@@ -49,6 +49,15 @@ __device__ __forceinline__ void adjoint(const Adj &P, int frame, int tr, int tc,
     const int col = c0 + C * lane, row = t0 + 2 * N * w;
     const int64_t hw = (int64_t)H * W;
 
+    if (EDGE && row >= H) {  // a warp below the frame only keeps the barriers
+        const float zero[C] = {};
+        sm.u.put(w, lane, zero);
+        for (int k = P.U - 1; k >= 0; --k) {
+            __syncthreads();
+            if (k > 0) __syncthreads();
+        }
+        return;
+    }
     const Cells<C, N, MODE> X(t0, row, col, H, W);
     // the row below a thread's rows (past an inner window's last: any row, it
     // is halo)
@@ -142,7 +151,7 @@ __device__ __forceinline__ void adjoint(const Adj &P, int frame, int tr, int tc,
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             f2 left_lane = shfl_up(gc[j][C - 1]);
-            if (EDGE && lane == 0) left_lane.v = 0ull;  // column -1, or halo
+            if (lane == 0) left_lane.v = 0ull;  // column -1, or halo
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const f2 up = j > 0 ? gr[j > 0 ? j - 1 : 0][c] : mk2(above[c], lo(gr[N - 1][c]));
@@ -184,7 +193,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_tv_adjoint(Adj P) {
     const int tc = (int)(blockIdx.x - t * (unsigned)P.nbands);
     const int frame = (int)(t / (unsigned)P.nchunks);
     const int tr = (int)(t - (unsigned)frame * (unsigned)P.nchunks);
-    const bool edge = tr == 0 || tr == P.nchunks - 1 || tc == 0 || tc == P.nbands - 1;
+    const bool edge = tr == P.nchunks - 1 || tc == P.nbands - 1;
     if (P.vec < 0) adjoint<C, N, NW, EDGE_WIDE>(P, frame, tr, tc, sm);
     else if (!P.vec) adjoint<C, N, NW, EDGE_SCALAR>(P, frame, tr, tc, sm);
     else if (edge) adjoint<C, N, NW, EDGE_VEC>(P, frame, tr, tc, sm);

@@ -254,7 +254,8 @@ struct Smem {
 // of `frame`.  PIN: start from p_a (P.p_in).  OUT_U: write u (and resid,
 // with PROJ 3 t = u + (u - f)), else p (P.p_out).  ENERGY: add the pass's
 // energy sums.  TAPE: also write every p_k (as 4 p) and, for k < nup, u_k
-// (P.tape_p, P.tape_u).  EDGE: the window touches a frame edge.
+// (P.tape_p, P.tape_u).  EDGE: the window reaches
+// the frame's last row or column.
 template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ, bool TAPE, int MODE>
 __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, int nup,
                                     Smem<C, NW> &sm) {
@@ -275,6 +276,22 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
     const bool bottom = cols && row + N >= own_r0 && row + N < own_r1;
     const Cells<C, N, MODE> X(t0, row, col, H, W);
     auto store = [&](float *plane, const f2 (&v)[N][C]) { X.store(plane, v, top, bottom); };
+
+    // A warp below the frame only keeps the barriers; the warp above reads
+    // zeros from it.
+    if (EDGE && row >= H) {
+        const float zero[C] = {};
+        sm.u.put(w, lane, zero);
+        for (int k = 1; k <= nup; ++k) {
+            __syncthreads();
+            if (OUT_U || k < nup) __syncthreads();
+        }
+        if (ENERGY) {
+            if (lane < SMAX) sm.energy[lane][w] = 0.f;
+            __syncthreads();
+        }
+        return;
+    }
 
     f2 f[N][C], u[N][C], pr[N][C], pc[N][C];
     // ---- input rows
@@ -306,9 +323,7 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             f2 left = shfl_up(pc[j][C - 1]);
-            if (EDGE || PIN) {
-                if (lane == 0) left = left0[j];
-            }
+            if (lane == 0) left = left0[j];
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const f2 up = j > 0 ? pr[j > 0 ? j - 1 : 0][c] : mk2(above[c], lo(pr[N - 1][c]));
@@ -327,7 +342,9 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
         const float *pb = P.p_in + (int64_t)frame * 2 * hw;
         float above[C];
         f2 left0[N];
-        X.load(pb, X.at(max(row - 1, 0), col, max(t0 - 1, 0), H, W), row > 0, above);
+        X.load(pb, X.at(max(row - 1, 0), col, max(t0 - 1, 0), H, W), true, above);
+#pragma unroll
+        for (int c = 0; c < C; ++c) above[c] = row > 0 ? above[c] : 0.f;
         const unsigned lo0 = (unsigned)max(c0 - 1, 0);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
@@ -452,7 +469,8 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
 template <int C, int N, int NW, bool PIN, bool OUT_U, bool ENERGY, int PROJ, bool TAPE = false>
 __device__ __forceinline__ void run_mode(const Pass &P, int frame, int tr, int tc, int nup,
                                          Smem<C, NW> &sm) {
-    const bool edge = tr == 0 || tr == P.nchunks - 1 || tc == 0 || tc == P.nbands - 1;
+    // the first windows of an axis need no bounds: they start at 0
+    const bool edge = tr == P.nchunks - 1 || tc == P.nbands - 1;
     if (TAPE && P.vec < 0) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, TAPE ? EDGE_WIDE : EDGE_SCALAR>(P, frame, tr, tc, nup, sm);
     else if (!P.vec) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, EDGE_SCALAR>(P, frame, tr, tc, nup, sm);
     else if (edge) run<C, N, NW, PIN, OUT_U, ENERGY, PROJ, TAPE, EDGE_VEC>(P, frame, tr, tc, nup, sm);

@@ -88,30 +88,49 @@ __global__ void k_cassi_phisum(const float *__restrict__ phi, float *__restrict_
     }
 }
 
-// detector grid: yb = A(x); ACC: y1 += y - yb, r = (y1 - yb)/ps; else r = (y - yb)/ps
+// detector grid (a block of a row per blockIdx, rows by blockIdx.y): yb = A(x);
+// ACC: y1 += y - yb, r = (y1 - yb)/ps; else r = (y - yb)/ps.  Eight bands'
+// loads in flight at a time; with an index division per pixel and a serial
+// loop over the bands left over by its unrolling it took 10 us at 256 x 256 x
+// 28 against XXX.
 template <bool ACC>
-__global__ void k_cassi_resid(const float *__restrict__ x, const float *__restrict__ phi,
-                              const float *__restrict__ y, float *__restrict__ y1,
-                              const float *__restrict__ ps, float *__restrict__ r, int L, int H,
-                              int W, int step) {
+__global__ void __launch_bounds__(128) k_cassi_resid(
+    const float *__restrict__ x, const float *__restrict__ phi, const float *__restrict__ y,
+    float *__restrict__ y1, const float *__restrict__ ps, float *__restrict__ r, int L, int H,
+    int W, int step, double *__restrict__ zero, int nzero) {
+    constexpr int G = 8;
+    grid_dep_wait();
+    if (blockIdx.x == 0 && blockIdx.y == 0)  // the next TV pass's stop-test sums
+        for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0.0;
     const int Wd = W + step * (L - 1);
-    const int64_t hw = (int64_t)H * W, n = (int64_t)H * Wd;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int h = (int)(i / Wd), wd = (int)(i - (int64_t)h * Wd);
-        int b0, b1;
-        band_range(wd, W, L, step, b0, b1);
+    const int64_t hw = (int64_t)H * W;
+    const int wd = blockIdx.x * blockDim.x + threadIdx.x;
+    if (wd >= Wd) return;
+    int b0, b1;
+    band_range(wd, W, L, step, b0, b1);
+    for (int h = blockIdx.y; h < H; h += gridDim.y) {
+        const int64_t i = (int64_t)h * Wd + wd;
+        const float yv = y[i], pv = ps[i], tv = ACC ? y1[i] : 0.f;
+        const float *xp = x + (int64_t)h * W + wd, *mp = phi + (int64_t)h * W + wd;
         float s = 0.f;
-        for (int b = b0; b <= b1; ++b) {
-            const int64_t p = (int64_t)h * W + (wd - step * b);
-            s = fmaf(__ldg(x + b * hw + p), __ldg(phi + p), s);
+        for (int b = b0; b <= b1; b += G) {
+            float xv[G], m[G];
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (b + u <= b1) {
+                    xv[u] = __ldg(xp + (b + u) * (hw - step));
+                    m[u] = __ldg(mp - (b + u) * step);
+                }
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (b + u <= b1) s = fmaf(xv[u], m[u], s);
         }
         if (ACC) {
-            const float t = y1[i] + (y[i] - s);
+            const float t = tv + (yv - s);
             y1[i] = t;
-            r[i] = __fdiv_rn(t - s, ps[i]);
+            r[i] = __fdiv_rn(t - s, pv);
         } else {
-            r[i] = __fdiv_rn(y[i] - s, ps[i]);
+            r[i] = __fdiv_rn(yv - s, pv);
         }
     }
 }
@@ -176,6 +195,10 @@ __global__ void __launch_bounds__(1024) k_cassi_proj_rows(
     }
 }
 
+dim3 resid_grid(int64_t Wd, int64_t H) {
+    return dim3((unsigned)((Wd + 127) / 128), (unsigned)std::min<int64_t>(H, 65535));
+}
+
 constexpr size_t kRowSmemMax = 48 * 1024;  // default dynamic shared memory limit
 
 // Projection form (SCI_CASSI_ROWS; bitwise the same result): 1, the
@@ -213,6 +236,11 @@ int tv_launch_flags(const float *f, float *u, float *resid, int64_t nf, int64_t 
                     void *workspace, size_t ws_bytes, cudaStream_t s, int force_R, int flags);
 double *tv_clear_region(int64_t nf, int64_t H, int64_t W, int K, void *workspace, int *words);
 size_t tv_workspace_bytes(int64_t nf, int64_t H, int64_t W, int K);
+bool tv_cassi_supported(int64_t L, int64_t H, int64_t W, int K);
+int tv_launch_cassi(const float *x, float *u, int64_t L, int64_t H, int64_t W, float weight,
+                    float eps, int K, int *steps, void *workspace, size_t ws_bytes,
+                    cudaStream_t s, int flags, const float *phi, const float *r, int detector,
+                    int step, float lam);
 
 static size_t r256(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -301,8 +329,42 @@ int sci_cassi_gap_tv(const float *y, const float *phi, const float *phisum, cons
     // the row-fused projection also clears the TV pass's stop-test sums, so
     // that the TV kernel follows it directly (flags 4)
     int nzero = 0;
+    // fused: the residual alone, on the detector grid, and the TV pass applies
+    // the projection as it loads x, which ping-pongs between x_out and xp
+    const bool fused = rows && tv_cassi_supported(L, H, W, o->tv_iter_max);
     double *zero = rows ? tv_clear_region(L, H, W, o->tv_iter_max, tv, &nzero) : nullptr;
+    auto enqueue_fused = [&](cudaStream_t s) -> int {
+        const int Wd = (int)(W + step * (L - 1));
+        float *X[2] = {x_out, xp};
+        const int start = o->iters & 1;  // the last iterate lands in x_out
+        if (x0 != X[start])
+            SCI_CUDA(cudaMemcpyAsync(X[start], x0, 4 * n, cudaMemcpyDeviceToDevice, s));
+        if (o->accelerate) SCI_CUDA(cudaMemsetAsync(y1, 0, 4 * nd, s));
+        if (o->sqerr) SCI_CUDA(cudaMemsetAsync(o->sqerr, 0, sizeof(double) * o->iters, s));
+        for (int it = 0; it < o->iters; ++it) {
+            SCI_CHECK_ARG(o->weights[it] > 0.f, "sci_cassi_gap_tv: tv_weight must be > 0");
+            const float *cur = X[(start + it) & 1];
+            float *nxt = X[(start + it + 1) & 1];
+            const dim3 g = resid_grid(Wd, H);
+            if (o->accelerate)
+                SCI_CUDA(launch_dep(k_cassi_resid<true>, g, dim3(128), 0, s, cur, phi, y, y1,
+                                    phisum, r, (int)L, (int)H, (int)W, step, zero, nzero));
+            else
+                SCI_CUDA(launch_dep(k_cassi_resid<false>, g, dim3(128), 0, s, cur, phi, y, y1,
+                                    phisum, r, (int)L, (int)H, (int)W, step, zero, nzero));
+            int e = tv_launch_cassi(cur, nxt, L, H, W, o->weights[it], o->eps, o->tv_iter_max,
+                                    o->tv_steps ? o->tv_steps + (int64_t)it * L : nullptr, tv,
+                                    tvb, s, 4, phi, r, Wd, step, o->lambdas[it]);
+            if (e) return e;
+            if (o->orig && o->sqerr) {
+                e = sci_sqerr_accum(o->orig, nxt, n, o->sqerr + it, s);
+                if (e) return e;
+            }
+        }
+        return SCI_OK;
+    };
     auto enqueue = [&](cudaStream_t s) -> int {
+        if (fused) return enqueue_fused(s);
         if (x0 != x_out) SCI_CUDA(cudaMemcpyAsync(x_out, x0, 4 * n, cudaMemcpyDeviceToDevice, s));
         if (o->accelerate) SCI_CUDA(cudaMemsetAsync(y1, 0, 4 * nd, s));
         if (o->sqerr) SCI_CUDA(cudaMemsetAsync(o->sqerr, 0, sizeof(double) * o->iters, s));
@@ -321,11 +383,11 @@ int sci_cassi_gap_tv(const float *y, const float *phi, const float *phisum, cons
                 SCI_LAUNCHED("k_cassi_proj_rows");
             } else {
                 if (o->accelerate)
-                    k_cassi_resid<true><<<grid1(nd, 256), 256, 0, s>>>(
-                        x_out, phi, y, y1, phisum, r, (int)L, (int)H, (int)W, step);
+                    k_cassi_resid<true><<<resid_grid(W + step * (L - 1), H), 128, 0, s>>>(
+                        x_out, phi, y, y1, phisum, r, (int)L, (int)H, (int)W, step, nullptr, 0);
                 else
-                    k_cassi_resid<false><<<grid1(nd, 256), 256, 0, s>>>(
-                        x_out, phi, y, y1, phisum, r, (int)L, (int)H, (int)W, step);
+                    k_cassi_resid<false><<<resid_grid(W + step * (L - 1), H), 128, 0, s>>>(
+                        x_out, phi, y, y1, phisum, r, (int)L, (int)H, (int)W, step, nullptr, 0);
                 SCI_LAUNCHED("k_cassi_resid");
                 k_cassi_update<<<grid1(n, 256), 256, 0, s>>>(x_out, phi, r, xp, o->lambdas[it],
                                                              (int)L, (int)H, (int)W, step);

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
         const int64_t p = (rev ? n4 - 1 - q : q) << 2;  // rev: bottom rows first
         const uint4 w = M.word4(p);
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 8
         for (int b = 0; b < B; ++b) {
             const float4 a = ldg4(x + b * hw + p), m = M.at4(b, p, w);
             s.x = fmaf(a.x, m.x, s.x);
@@ -434,7 +434,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
         const int64_t p = (rev ? n4 - 1 - q : q) << 2;
         const uint4 w = M.word4(p);
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 8
         for (int b = 0; b < B; ++b) {
             const float4 m = M.at4(b, p, w);
             const float4 t = tload(b * hw + p);
@@ -653,6 +653,14 @@ int proj_gap_rn(const float *x, const float *phi, const uint32_t *mask_bits, con
     return SCI_OK;
 }
 
+// Threads per block of the residual passes (4 pixels each): 256, or fewer where
+// 256 would leave SMs without a block.
+static int resid_threads(int64_t hw) {
+    int t = 256;
+    while (t > 64 && hw / 4 < (int64_t)kSMs * 2 * t) t >>= 1;
+    return t;
+}
+
 int gap_residual_rn(const float *x, const float *phi, const uint32_t *mask_bits,
                      const float *y, float *y1, const float *phisum, float *c,
                      int accelerate, int64_t B, int64_t H, int64_t W, void *stream, double *rn,
@@ -665,18 +673,19 @@ int gap_residual_rn(const float *x, const float *phi, const uint32_t *mask_bits,
     SCI_CHECK_ARG(vec_ok(hw, {x, phi, mask_bits, y, y1, phisum, c}),
                   "sci_gap_residual: needs H*W %% 4 == 0 and 16-byte aligned buffers");
     cudaStream_t s = as_stream(stream);
-    const dim3 g = grid_for(hw / 4, 256);
+    const int T = resid_threads(hw);
+    const dim3 g = grid_for(hw / 4, T);
     if (mask_bits) {
         Mask<1> M{mask_bits, hw};
-        if (accelerate) SCI_CUDA(launch_dep(k_gap_resid_vec<1, true>, g, dim3(256), 0, s, x, M, y, y1,
+        if (accelerate) SCI_CUDA(launch_dep(k_gap_resid_vec<1, true>, g, dim3(T), 0, s, x, M, y, y1,
                                         phisum, c, (int)B, hw, rn, zero, nzero, resid_rev()));
-        else SCI_CUDA(launch_dep(k_gap_resid_vec<1, false>, g, dim3(256), 0, s, x, M, y, y1,
+        else SCI_CUDA(launch_dep(k_gap_resid_vec<1, false>, g, dim3(T), 0, s, x, M, y, y1,
                                         phisum, c, (int)B, hw, rn, zero, nzero, resid_rev()));
     } else {
         Mask<0> M{phi, hw};
-        if (accelerate) SCI_CUDA(launch_dep(k_gap_resid_vec<0, true>, g, dim3(256), 0, s, x, M, y, y1,
+        if (accelerate) SCI_CUDA(launch_dep(k_gap_resid_vec<0, true>, g, dim3(T), 0, s, x, M, y, y1,
                                         phisum, c, (int)B, hw, rn, zero, nzero, resid_rev()));
-        else SCI_CUDA(launch_dep(k_gap_resid_vec<0, false>, g, dim3(256), 0, s, x, M, y, y1,
+        else SCI_CUDA(launch_dep(k_gap_resid_vec<0, false>, g, dim3(T), 0, s, x, M, y, y1,
                                         phisum, c, (int)B, hw, rn, zero, nzero, resid_rev()));
     }
     SCI_LAUNCHED("k_gap_resid");
@@ -697,10 +706,11 @@ int admm_residual_rn(const float *t, const uint32_t *mask_bits, const float *y,
     SCI_CHECK_ARG(vec_ok(hw, {t, mask_bits, y, phisum, r_new, x_out}),
                   "admm residual: needs H*W %% 4 == 0 and 16-byte aligned buffers");
     cudaStream_t s = as_stream(stream);
-    const dim3 g = grid_for(hw / 4, 256);
+    const int T = resid_threads(hw);
+    const dim3 g = grid_for(hw / 4, T);
     Mask<1> M{mask_bits, hw};
 #define SCI_ADMM_RESID(F, X)                                                                  \
-    SCI_CUDA(launch_dep(k_admm_resid_vec<F, X>, g, dim3(256), 0, s, t, M, y, phisum, r_new,   \
+    SCI_CUDA(launch_dep(k_admm_resid_vec<F, X>, g, dim3(T), 0, s, t, M, y, phisum, r_new,   \
                         x_out, lambda, gamma, (int)B, hw, rn, zero, nzero, resid_rev()))
     if (first) {
         if (x_out) SCI_ADMM_RESID(true, true);

@@ -227,6 +227,8 @@ struct RuleArgs {
     // the on-load projection's mask as floats, one plane per frame, instead of
     // packed (the lean pass and the tiles)
     const float *phi = nullptr;
+    // the spectral on-load projection (tiles): detector columns, columns per band
+    int detector = 0, step = 0;
 };
 
 static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, int64_t H,
@@ -302,11 +304,13 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
                       (!ra.tout || (reinterpret_cast<uintptr_t>(ra.tout) % (4 * cpl_pick)) == 0);
     SCI_CHECK_ARG(!ra.tout || (proj && slim), "tv: the t output needs the lean pass with the "
                                               "on-load projection (aligned frames)");
-    const int pmode = proj ? (ra.tout ? 3 : (ra.phi ? 2 : 1)) : 0;  // the lean pass's PROJ
+    const int pmode = !proj ? 0 : ra.detector ? 5 : ra.tout ? 3 : ra.phi ? 2 : 1;  // the lean pass's PROJ
     // the clip rule in one pass on the lean pipeline (4 columns per lane)
     const bool clip = slim_enabled() && ra.rule == RULE_CLIP && !resid && U <= SMAX &&
                       force_R <= 0 && !getenv("SCI_TV_R") && aligned_for(4);
-    SCI_CHECK_ARG(!proj || slim || clip || !(ra.phi || ra.rule == RULE_CLIP),
+    SCI_CHECK_ARG(!ra.detector || use_tiles(nf, H, W, slim),
+                  "tv: the spectral on-load projection needs tiles");
+    SCI_CHECK_ARG(!proj || ra.detector || slim || clip || !(ra.phi || ra.rule == RULE_CLIP),
                   "tv: this on-load projection needs the lean pass (aligned frames)");
     const int cpl = slim ? cpl_pick : ((proj || ra.rule != RULE_SKIMAGE) ? 4 : cpl_pick);
     const bool vec = (W % cpl == 0) && (fs % cpl == 0) &&
@@ -359,6 +363,8 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
         P.bits = proj_bits;
         P.cmap = proj_c;
         P.phi = ra.phi;
+        P.frame0 = ra.detector;
+        P.B = ra.step;
         P.lam = proj_lam;
         P.frame_fast = frame_fast_order(proj);
         P.nbands = band_count((int)W, 32 * cpl, P.hl, P.hr);
@@ -438,6 +444,28 @@ int tv_launch_phi(const float *f, float *u, int64_t nf, int64_t H, int64_t W, in
     ra.phi = phi;
     return tv_launch_core(f, u, nullptr, nf, H, W, fs, weight, eps, K, steps, nullptr, workspace,
                           ws_bytes, s, 0, flags, nullptr, proj_c, proj_lam, ra);
+}
+
+// Whether the spectral solver's TV can apply the projection as it loads x (K
+// as n_iter_max): where the tiles are the faster pass.
+bool tv_cassi_supported(int64_t L, int64_t H, int64_t W, int K) {
+    const char *e = getenv("SCI_FUSED_PROJ");
+    return !(e && atoi(e) == 0) && slim_enabled() && K >= 2 && K <= tv::SMAX + 1 &&
+           H * W < (int64_t(1) << 30) && use_tiles(L, H, W, true);
+}
+
+// tv_launch_impl with x + lam (r[h, w + step b] phi[h, w]) applied as x is
+// loaded (r: H x detector).
+int tv_launch_cassi(const float *x, float *u, int64_t L, int64_t H, int64_t W, float weight,
+                    float eps, int K, int *steps, void *workspace, size_t ws_bytes,
+                    cudaStream_t s, int flags, const float *phi, const float *r, int detector,
+                    int step, float lam) {
+    RuleArgs ra;
+    ra.phi = phi;
+    ra.detector = detector;
+    ra.step = step;
+    return tv_launch_core(x, u, nullptr, L, H, W, H * W, weight, eps, K, steps, nullptr, workspace,
+                          ws_bytes, s, 0, flags, nullptr, r, lam, ra);
 }
 
 // tv_launch_impl with the on-load projection that also stores t = u + (u -

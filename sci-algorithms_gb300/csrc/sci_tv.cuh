@@ -107,7 +107,9 @@ struct Pass {
     int early;            // more blocks than fit at once: grid_dep_launch()
     // phi: a float mask, one plane per frame (the lean pass's PROJ 2, tiles'
     // 4).  Unrolled solver (tiles' PROJ 2): frames are frames frame0 .. of N
-    // scenes of B; f holds x, cmap the scenes' maps q, phi [B][H][W].
+    // scenes of B; f holds x, cmap the scenes' maps q, phi [B][H][W].  Spectral
+    // projection (tiles' 5): cmap [H][frame0], band b's columns from B b on; phi
+    // [H][W].
     const float *phi, *lam_dev;
     int frame0, B;
 };

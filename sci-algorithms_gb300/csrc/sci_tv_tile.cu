@@ -58,10 +58,11 @@ int tile_columns() { return C; }
 int64_t tile_blocks(const Pass &P) { return (int64_t)P.nbands * P.nchunks * P.nf; }
 int tile_resident_blocks() { return MINB; }
 
-// proj as launch_slim's
+// proj as launch_slim's, 5 the spectral projection
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s) {
     if (proj == 3) main_pass<false, true, 3>(P, s);
     else if (proj == 2) main_pass<false, true, 4>(P, s);
+    else if (proj == 5) main_pass<false, true, 5>(P, s);
     else if (proj) main_pass<false, true, 1>(P, s);
     else if (!pin && final_pass) main_pass<false, true, 0>(P, s);
     else if (!pin) main_pass<false, false, 0>(P, s);
@@ -72,6 +73,7 @@ void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_
 void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s) {
     if (proj == 3) fix_pass<false, 3>(P, s);
     else if (proj == 2) fix_pass<false, 4>(P, s);
+    else if (proj == 5) fix_pass<false, 5>(P, s);
     else if (proj) fix_pass<false, 1>(P, s);
     else if (pin) fix_pass<true, 0>(P, s);
     else fix_pass<false, 0>(P, s);

@@ -176,14 +176,14 @@ struct Cells {
 
 // One row of the input f of a frame (its stack at fb): the stored values, or
 // with the projection applied as it is loaded -- PROJ 1, 3: a packed binary
-// mask (proj_px); PROJ 4: a float mask; PROJ 2: the unrolled solver's v = x + lam (q phi_b), with a
+// mask (proj_px); PROJ 4: a float mask; PROJ 5: the spectral projection; PROJ 2: the unrolled solver's v = x + lam (q phi_b), with a
 // float mask per frame of a scene, the map q per scene and lam in device
 // memory.
 template <int PROJ, int C, int N, int MODE, typename Args>
 __device__ __forceinline__ void load_f(const Args &P, const Cells<C, N, MODE> &X,
                                        const float *fb, int frame,
                                        typename Cells<C, N, MODE>::Off o, bool in,
-                                       float (&v)[C]) {
+                                       float (&v)[C], int row = 0, int col = 0) {
     X.load(fb, o, in, v);
     if constexpr (PROJ == 1 || PROJ == 3) {
         float cm[C], wb[C];
@@ -192,6 +192,16 @@ __device__ __forceinline__ void load_f(const Args &P, const Cells<C, N, MODE> &X
 #pragma unroll
         for (int c = 0; c < C; ++c)
             v[c] = proj_px(P.lam, cm[c], v[c], __float_as_uint(wb[c]), 1u << frame);
+    } else if constexpr (PROJ == 5) {
+        // one aperture for all bands, the map on the detector: band b's columns
+        // lie B b to the right in rows of frame0 columns (scalars: any step)
+        const float *q = P.cmap + (int64_t)(MODE == INSIDE ? row : min(row, P.H - 1)) * P.frame0 +
+                         P.B * frame;
+        float m[C];
+        X.load(P.phi, o, in, m);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            v[c] = fmaf(P.lam, q[MODE == INSIDE ? col + c : min(col + c, P.W - 1)] * m[c], v[c]);
     } else if constexpr (PROJ == 4) {
         float q[C], m[C];
         X.load(P.cmap, o, in, q);
@@ -300,7 +310,7 @@ __device__ __forceinline__ void run(const Pass &P, int frame, int tr, int tc, in
         float v[2][C];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            load_f<PROJ>(P, X, fb, frame, X.off[h][j], X.inside(h, j), v[h]);
+            load_f<PROJ>(P, X, fb, frame, X.off[h][j], X.inside(h, j), v[h], row + j + h * N, col);
         }
 #pragma unroll
         for (int c = 0; c < C; ++c) {

@@ -109,3 +109,28 @@ def test_cassi_row_projection_and_graph_are_bitwise_equal(monkeypatch, accelerat
             out.append(s.run(yd).clone())  # replay of the cached graph
     for o in out[1:]:
         assert torch.equal(o, out[0])
+
+
+@pytest.mark.parametrize("H,W,L,step", [(1, 2, 3, 1), (7, 9, 4, 2), (48, 64, 5, 3), (49, 65, 6, 2),
+                                        (88, 121, 3, 1), (90, 132, 28, 2)])
+@pytest.mark.parametrize("accelerate,eps,iters", [(True, 2e-4, 4), (False, 0.05, 5)])
+def test_cassi_projection_on_load_is_bitwise_equal(monkeypatch, H, W, L, step, accelerate, eps,
+                                                   iters):
+    """The residual kernel with the projection applied as the TV tiles load x
+    against the projection kernel and the plain TV: the same operations.
+    Sizes around the tiles' 64 x 48 windows, odd widths and steps (unaligned
+    detector columns), stops inside the pass (eps = 0.05), odd and even
+    iteration counts (the stack ping-pongs)."""
+    rng = np.random.default_rng(H * W + L)
+    phi = torch.from_numpy(rng.random((H, W)).astype(np.float32)).cuda()
+    op = sci.CassiOperator(phi, L, step)
+    y = torch.from_numpy(rng.random((H, op.Wd)).astype(np.float32)).cuda()
+    out = []
+    for fused in ("0", "1"):
+        monkeypatch.setenv("SCI_FUSED_PROJ", fused)
+        for graph in (False, True):
+            s = sci.CassiSolver(op, iters, 0.8, 0.1, 5, eps=eps, accelerate=accelerate,
+                                use_graph=graph)
+            out.append(s.run(y).clone())
+    for x in out[1:]:
+        assert torch.equal(out[0], x)

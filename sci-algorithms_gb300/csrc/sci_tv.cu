@@ -389,7 +389,6 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
             const int c = tile_columns();
             P.vec = aligned_for(c) && reinterpret_cast<uintptr_t>(ra.tout) % (4 * c) == 0;
             tile_geometry(P);
-            P.early = tile_blocks(P) > kSMs * tile_resident_blocks();
             launch_tile(P, PIN, FINAL, pmode, s);
         } else if (clip) {
             P.early = pass_blocks(P) > (unsigned)(kSMs * clip_resident_blocks());

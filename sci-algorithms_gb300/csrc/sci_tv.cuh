@@ -841,26 +841,28 @@ __device__ __forceinline__ bool decode_item(const Pass &P, int &frame, int &chun
 
 // First j in this pass's window with |E_{j-1} - E_j| < eps * E_0, or -1.
 // CG: read the sums from L2 (they were added by other blocks' atomics
-// during the same launch).
+// during the same launch).  All of the window's sums are loaded before the
+// first is looked at: one after the other they were five round trips to L2
+// at the end of every pass.
 template <bool CG = false>
 __device__ __forceinline__ int find_stop(const Pass &P, int frame) {
     const int SG = P.S;
     const double *eb = P.energy + (int64_t)frame * P.K * 2;
     auto ld = [&](int i) { return CG ? __ldcg(eb + i) : eb[i]; };
     const double inv = 1.0 / ((double)P.H * (double)P.W);
-    const double w = (double)P.weight;
     const int j0 = max(1, P.a), j1 = min(P.a + SG - 1, P.K - 2);
     if (j0 > j1) return -1;
-    const double e0 = (ld(0) + w * ld(1)) * inv;
-    double eprev = (ld(2 * (j0 - 1)) + w * ld(2 * (j0 - 1) + 1)) * inv;
-    for (int j = j0; j <= j1; ++j) {
-        const double e = (ld(2 * j) + w * ld(2 * j + 1)) * inv;
-        if (fabs(eprev - e) < (double)P.eps * e0) return j;
-        eprev = e;
-    }
-    return -1;
+    const double e0 = ld(0);
+    double e[SMAX + 1];  // E_{j0-1} ..; the window holds at most SMAX + 1 sums
+#pragma unroll
+    for (int q = 0; q <= SMAX; ++q) e[q] = ld(2 * min(j0 - 1 + q, j1));
+    int stop = -1;
+#pragma unroll
+    for (int q = 1; q <= SMAX; ++q)
+        if (stop < 0 && j0 - 1 + q <= j1 && fabs(e[q - 1] * inv - e[q] * inv) < (double)P.eps * (e0 * inv))
+            stop = j0 - 1 + q;
+    return stop;
 }
-
 template <int CPL>
 constexpr int min_blocks() { return CPL == 2 ? 4 : 3; }
 

@@ -7,26 +7,26 @@
 // 24.7 / 26.3 / 63.6 / 745; 4 at 96 23.9 / 25.6 / 59.5 / 645; 2 x 4 pixels,
 // 8 warps at 64 24.7 / 26.1 / 67.1 / 719.  Warps in flight count for more
 // than the last spills.
-#include "sci_tv_tile.cuh"
+#include "sci_tv_tile_launch.cuh"
 
 namespace sci {
 namespace tv {
 
+void tile_small_geometry(Pass &P);  // sci_tv_tile_small.cu
+void launch_tile_small(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s);
+void launch_tile_small_fix(const Pass &P, bool pin, int proj, cudaStream_t s);
+
 namespace {
-constexpr int C = 2, N = 4, NW = 6, MINB = 4;
+using Large = tile::Shape<2, 4, 6, 4>;
 
-dim3 blocks(const Pass &P) { return dim3((unsigned)tile_blocks(P)); }
-
-template <bool PIN, bool OUT_U, int PROJ>
-void main_pass(const Pass &P, cudaStream_t s) {
-    (void)launch_dep(tile::k_tv_tile<C, N, NW, MINB, PIN, OUT_U, PROJ>, blocks(P), dim3(NW * 32),
-                     0, s, P);  // reported by the caller's cudaGetLastError
-}
-template <bool PIN, int PROJ>
-void fix_pass(const Pass &P, cudaStream_t s) {
-    (void)launch_dep(tile::k_tv_tile_fix<C, N, NW, MINB, PIN, PROJ>, blocks(P), dim3(NW * 32), 0,
-                     s, P);
-}
+// Fewer windows than fill the GPU's 608 slots: half the pixels per thread, so
+// that a window's chain of updates is shorter and there are more warps to
+// overlap.  Measured (TV call with its memset and stop-test launch, large /
+// small windows, us): 8 x 64 x 96 (32 windows of the large shape) 11.9 / 10.4,
+// 8 x 256 x 256 (280) 14.5 / 12.6, 32 x 128 x 128 (384) 14.5 / 14.6, 12 x 256
+// x 256 (420) 15.8 / 16.4, 16 x 256 x 256 (560) 16.5 / 16.7, 28 x 256 x 256
+// (980) 22.3 / 22.8, 24 x 512 x 512 (2808) 41.3 / 47.4.
+bool small(const Pass &P) { return Large::windows(P.nf, P.H, P.W) <= 300; }
 }  // namespace
 
 // Which calls run on tiles (slim: the lean row pipeline could run it, frames
@@ -43,40 +43,23 @@ void fix_pass(const Pass &P, cudaStream_t s) {
 //   x 517 x 643 161 / 259, 16 x 1024 x 1024 602 / 792, 24 x 2048 x 2048 3130
 //   / 2570.
 bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim) {
-    using G = tile::Geo<C, N, NW>;
-    return nf * tile::window_count((int)H, G::ROWS) * tile::window_count((int)W, G::COLS) <=
-           (slim ? 2000 : 14000);
+    return Large::windows(nf, H, W) <= (slim ? 2000 : 14000);
 }
 
-// Window counts and the pass's launches.
 void tile_geometry(Pass &P) {
-    using G = tile::Geo<C, N, NW>;
-    P.nchunks = tile::window_count(P.H, G::ROWS);
-    P.nbands = tile::window_count(P.W, G::COLS);
+    if (small(P)) tile_small_geometry(P);
+    else Large::geometry(P);
 }
-int tile_columns() { return C; }
-int64_t tile_blocks(const Pass &P) { return (int64_t)P.nbands * P.nchunks * P.nf; }
-int tile_resident_blocks() { return MINB; }
+int tile_columns() { return 2; }
 
-// proj as launch_slim's, 5 the spectral projection
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s) {
-    if (proj == 3) main_pass<false, true, 3>(P, s);
-    else if (proj == 2) main_pass<false, true, 4>(P, s);
-    else if (proj == 5) main_pass<false, true, 5>(P, s);
-    else if (proj) main_pass<false, true, 1>(P, s);
-    else if (!pin && final_pass) main_pass<false, true, 0>(P, s);
-    else if (!pin) main_pass<false, false, 0>(P, s);
-    else if (final_pass) main_pass<true, true, 0>(P, s);
-    else main_pass<true, false, 0>(P, s);
+    if (small(P)) launch_tile_small(P, pin, final_pass, proj, s);
+    else Large::launch(P, pin, final_pass, proj, s);
 }
 
 void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s) {
-    if (proj == 3) fix_pass<false, 3>(P, s);
-    else if (proj == 2) fix_pass<false, 4>(P, s);
-    else if (proj == 5) fix_pass<false, 5>(P, s);
-    else if (proj) fix_pass<false, 1>(P, s);
-    else if (pin) fix_pass<true, 0>(P, s);
-    else fix_pass<false, 0>(P, s);
+    if (small(P)) launch_tile_small_fix(P, pin, proj, s);
+    else Large::launch_fix(P, pin, proj, s);
 }
 
 }  // namespace tv

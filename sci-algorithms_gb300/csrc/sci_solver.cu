@@ -42,12 +42,12 @@ int proj_gap_rn(const float *x, const float *phi, const uint32_t *mask_bits, con
 int gap_residual_rn(const float *x, const float *phi, const uint32_t *mask_bits,
                     const float *y, float *y1, const float *phisum, float *c,
                     int accelerate, int64_t B, int64_t H, int64_t W, void *stream, double *rn,
-                    double *zero, int nzero);
+                    double *zero, int nzero, const float *orig, double *sq);
 double *tv_clear_region(int64_t nf, int64_t H, int64_t W, int K, void *workspace, int *words);
 int admm_residual_rn(const float *t, const uint32_t *mask_bits, const float *y,
                      const float *phisum, float *r_new, float *x_out, float lambda, float gamma,
                      int first, int64_t B, int64_t H, int64_t W, void *stream, double *rn,
-                     double *zero, int nzero);
+                     double *zero, int nzero, const float *orig, double *sq);
 int tv_launch_tout(const float *f, float *u, int64_t nf, int64_t H, int64_t W, int64_t fs,
                    float weight, float eps, int K, int *steps, void *workspace, size_t ws_bytes,
                    cudaStream_t s, int flags, const uint32_t *proj_bits, const float *proj_c,
@@ -177,6 +177,7 @@ int enqueue(const Args &a, cudaStream_t s) {
     if (o.resid_norm) SCI_CUDA(cudaMemsetAsync(o.resid_norm, 0, sizeof(double) * o.iters, s));
     // FP64 ||r||^2 of iteration `it`'s projection residual (nullable)
     auto rn = [&](int it) { return o.resid_norm ? o.resid_norm + it : nullptr; };
+    auto sq = [&](int it) { return o.sqerr ? o.sqerr + it : nullptr; };
     const bool aligned = ((reinterpret_cast<uintptr_t>(a.x0) | reinterpret_cast<uintptr_t>(a.x_out) |
                            reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.phisum) |
                            reinterpret_cast<uintptr_t>(a.bits) | (a.bits ? 0 : reinterpret_cast<uintptr_t>(a.phi))) & 15u) == 0;
@@ -203,8 +204,11 @@ int enqueue(const Args &a, cudaStream_t s) {
             const float *cur = X[(start + it) & 1];
             float *nxt = X[(start + it + 1) & 1];
             int *steps = o.tv_steps ? o.tv_steps + (int64_t)it * B : nullptr;
+            // the squared error of the iterate it starts from, but the first
+            const bool track = o.orig && o.sqerr && it > 0;
             int e = gap_residual_rn(cur, phi, a.bits, a.y, w.y1, a.phisum, w.c, o.accelerate, B,
-                                    H, W, s, rn(it), zero, nzero);
+                                    H, W, s, rn(it), zero, nzero, track ? o.orig : nullptr,
+                                    track ? o.sqerr + it - 1 : nullptr);
             if (e) return e;
             if (o.tvm)  // the clip files take tvweight itself
                 e = tvx_launch(o.tvm, cur, nxt, nullptr, B, H, W, o.weights[it], K, steps, w.tv,
@@ -217,7 +221,7 @@ int enqueue(const Args &a, cudaStream_t s) {
                                    nullptr, w.tv, w.tv_bytes, s, 0, 4, a.bits, w.c,
                                    o.lambdas[it]);
             if (e) return e;
-            if (o.orig && o.sqerr) {
+            if (o.orig && o.sqerr && it == o.iters - 1) {
                 e = sci_sqerr_accum(o.orig, nxt, n, o.sqerr + it, s);
                 if (e) return e;
             }
@@ -262,16 +266,13 @@ int enqueue(const Args &a, cudaStream_t s) {
             float *cur = T[it & 1], *nxt = T[(it + 1) & 1];
             int e = admm_residual_rn(it ? tb : cur, a.bits, a.y, a.phisum, R,
                                      want_x ? a.x_out : nullptr, o.lambdas[it], gamma, it == 0, B,
-                                     H, W, s, rn(it), zero, nzero);
+                                     H, W, s, rn(it), zero, nzero, o.orig,
+                                     o.orig ? sq(it) : nullptr);
             if (e) return e;
             e = tv_launch_tout(cur, nxt, B, H, W, hw, o.weights[it], o.eps, K,
                                o.tv_steps ? o.tv_steps + (int64_t)it * B : nullptr, w.tv,
                                w.tv_bytes, s, 4, a.bits, R, o.lambdas[it], tb);
             if (e) return e;
-            if (o.orig && o.sqerr) {
-                e = sci_sqerr_accum(o.orig, a.x_out, n, o.sqerr + it, s);
-                if (e) return e;
-            }
         }
         return SCI_OK;
     }

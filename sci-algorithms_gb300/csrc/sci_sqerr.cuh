@@ -76,6 +76,11 @@ struct SquareSum {
         c.add(lo(u), lo(ue));
         c.add(hi(u), hi(ue));
     }
+    __device__ __forceinline__ void add4(float4 a, float4 b) {
+        const float x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+        const float d[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
+        add4(x, y, d);
+    }
     __device__ __forceinline__ double take() {
         const double r = c.take() + wide;
         wide = 0.0;

@@ -45,10 +45,9 @@ int sci_last_error(char *buf, size_t n);
 /* Reads the device status word into *status and, with clear != 0, resets
  * it.  Bit 0 is set when a bounded device-side wait of a bulk-copy kernel
  * (the GAP projection of sci_proj_gap with a packed mask, the batched and
- * convolution kernels) gave up; bit 1 when a wait of the batched solve's
- * work queue (sci_batch_gap_tv) gave up.  The results of such a launch are
- * not valid.  Synchronous.  No counterpart in the reference (library
- * plumbing). */
+ * convolution kernels) gave up, and the results of such a launch are not
+ * valid; bit 1 by sci_batch_selftest_queue_wait.  Synchronous.  No
+ * counterpart in the reference (library plumbing). */
 int sci_device_status(unsigned int *status, int clear);
 
 /* Exercises the error path of the bounded device-side waits: one block
@@ -292,40 +291,33 @@ typedef struct sci_batch_item {
 int sci_batch_workspace_bytes(const sci_batch_item *items, int n, int tv_iter_max,
                               size_t *bytes);
 
-/* Autotuner of the batched solve: times candidate tilings on a few
+/* Autotuner of the batched solve: times candidate row-chunk heights on a few
  * iterations of the batch's own solve (from x0 = At(y / phisum), overwriting
- * every item's x) -- row-chunk heights of 1/2, 1 and 2 times the default for
- * each item's height, and 4 columns per lane for every item or 2 for items
- * at most 256 columns wide -- and writes the fastest into items[i].R and
- * items[i].cpl; with a non-null iters_per_launch it then times 1, 2 or 3
- * iterations per persistent launch against all of them and writes the
- * fastest (0: all in one launch).  Cached per process for the list of
+ * every item's x) -- those that make 1, 2, 3 or 6 waves of TV work items --
+ * and writes the fastest into items[i].R (and 4 into items[i].cpl).  A
+ * non-null iters_per_launch receives 0.  Cached per process for the list of
  * shapes.  Synchronises the stream. */
 int sci_batch_autotune(sci_batch_item *items, int n, int iters, int tv_iter_max,
                        float eps, int accelerate, int *iters_per_launch,
                        void *workspace, size_t workspace_bytes, void *stream);
 
 /* GAP-TV (pnp_sci_algo.py:536-706, denoiser='tv') of n <= 256 independent
- * measurements, all items advancing together: persistent launches over a
- * device work queue, each running iters_per_launch iterations (0: all) of
- * every item -- per iteration the projection tiles, TV work items and stop
- * tests of all items, a task waiting (bounded) only for earlier tasks of
- * its own item.  With use_graph the whole loop is captured once into a
- * cached CUDA graph.  init_x0: start from At(y / phisum) (else from x).
- * tv_iter_max in [2, 5].  The item table is uploaded synchronously before
- * the work is enqueued.  A wait that gave up sets bit 1 of the device
- * status (sci_device_status). */
+ * measurements, all items advancing together: per iteration one launch each
+ * for the residual maps, the TV work items and the stop tests of all items.
+ * With use_graph the whole loop is captured once into a cached CUDA graph.
+ * init_x0: start from At(y / phisum) (else from x).  tv_iter_max in [2, 5].
+ * The item table is uploaded synchronously before the work is enqueued.
+ * iters_per_launch (>= 0) has no effect. */
 int sci_batch_gap_tv(const sci_batch_item *items, int n, int iters,
                      int tv_iter_max, float eps, int accelerate, int init_x0,
                      int use_graph, int iters_per_launch, void *workspace,
                      size_t workspace_bytes, void *stream);
 
-/* Exercises the give-up path of the work queue's bounded waits: one warp
- * waits, `polls` times at most (1 .. 2^20), for a task count that nothing
- * raises, then raises the queue's abort flag, which sets bit 1 of the
- * device status word.  workspace: any device buffer of at least 4 KB (the
- * queue's counters are placed there).  For tests of that path; the context
- * stays usable.  No counterpart in the reference. */
+/* Exercises a bounded wait that gives up: one warp polls, `polls` times at
+ * most (1 .. 2^20), a count that nothing raises, then sets bit 1 of the device
+ * status word (sci_device_status).  workspace: any device buffer of at least
+ * 4 KB.  For tests; the context stays usable.  No counterpart in the
+ * reference. */
 int sci_batch_selftest_queue_wait(unsigned int polls, void *workspace,
                                   size_t workspace_bytes, void *stream);
 

@@ -2,15 +2,12 @@
 
 ``BatchSolver`` builds one device item table for a list of measurements
 (each with its own binary mask, packed to one word per pixel) and calls
-``sci_batch_gap_tv``: persistent launches over a device work queue run the
-projection tiles, TV work items and stop tests of every item, each task
-waiting only for earlier tasks of its own item, and the whole loop is
-captured once into a CUDA graph.  ``autotune=True`` lets
-``sci_batch_autotune`` pick each shape's TV column width and row-chunk
-height, and the iterations per persistent launch, by timing them on the
-items' data.  Each item's result equals a single-measurement
-``gap_denoise`` (``PnP_SCI/python/pnp_sci_algo.py:536``) with
-x0 = At(y / Phi_sum).
+``sci_batch_gap_tv``: per iteration one launch each for the residual maps,
+the TV work items and the stop tests of every item, the whole loop captured
+once into a CUDA graph.  ``autotune=True`` lets ``sci_batch_autotune`` pick
+the TV row-chunk heights by timing them on the items' data.  Each item's
+result equals a single-measurement ``gap_denoise``
+(``PnP_SCI/python/pnp_sci_algo.py:536``) with x0 = At(y / Phi_sum).
 """
 import ctypes
 
@@ -49,7 +46,7 @@ class BatchSolver:
         nb = ctypes.c_size_t()
         call("sci_batch_workspace_bytes", self.items, n, self.K, ctypes.byref(nb))
         self.ws = _dev.workspace(nb.value, self.dev)
-        # iterations per persistent launch of the work queue (0: all)
+        # accepted by sci_batch_gap_tv, without effect
         self.iters_per_launch = 0
         if autotune:
             self._call(0, 1, graph=False)  # x = x0, a realistic input to time on

@@ -4,20 +4,19 @@
 // (admmdenoise_cacti's frame-block loop, PnP_SCI/python/pnp_sci_algo.py:498);
 // here a batch of independent measurements (each with its own H x W x B and
 // packed binary mask) advances together.  Every phase of an iteration is
-// one launch over a work queue spanning all items: the GAP projection over
-// 256-pixel tiles of every item, then the Chambolle TV pass over every
-// item's (frame, row chunk, column band) tiles, then the stop-test launch
-// over the same tiles.  Items are found from the tile index through prefix
-// tables in a device-resident item table.  The whole multi-iteration loop is
-// captured once into a CUDA graph and replayed.  An autotuner times the TV
-// row-chunk height per distinct frame shape on the item's own data.
+// one launch spanning all items: the GAP residual maps, then the Chambolle
+// TV pass over every item's (frame, row chunk, column band) work items, then
+// the stop-test launch over the same work items (sci_batch_lean.cu).  Items
+// are found from the task index through prefix tables in a device-resident
+// item table.  The whole multi-iteration loop is captured once into a CUDA
+// graph and replayed.  An autotuner times row-chunk heights on the batch's
+// own data.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
-#include <tuple>
 #include <vector>
 
 #include "sci_bulk.cuh"
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(tv::WPB * 32, 3) k_batch_tv(const Table *__res
 size_t r256(size_t b) { return (b + 255) & ~size_t(255); }
 
 struct Layout {
-    size_t table, xp, y1, energy, stop, queue, tvscratch, total;
+    size_t table, xp, y1, energy, stop, tvscratch, total;
     std::vector<size_t> item_xp, item_y1, item_c, item_e, item_e1, item_stop;
 };
 
@@ -217,7 +216,7 @@ Layout layout(const sci_batch_item *items, int n, int K) {
         L.item_c.push_back(off);
         off += r256(4 * (size_t)hw);
     }
-    // per item the energy sums of even and odd iterations (the per-phase
+    // per item the energy sums of even and odd iterations (the generic
     // launches use the first), then its stop decisions and ticket
     L.energy = off;
     for (int i = 0; i < n; ++i) {
@@ -226,23 +225,22 @@ Layout layout(const sci_batch_item *items, int n, int K) {
         L.item_e1.push_back(off + eb - L.energy);
         off += 2 * eb;
     }
-    const size_t energy_end = off;
     L.stop = off;
     for (int i = 0; i < n; ++i) {
         L.item_stop.push_back(off);
         off += r256(sizeof(int) * (size_t)items[i].B + sizeof(unsigned));
     }
-    L.queue = off;
-    off += r256(sizeof(Queue));
     L.tvscratch = off;
     size_t tvmax = 0;  // autotuning scratch: the largest single-item TV workspace
     for (int i = 0; i < n; ++i)
         tvmax = std::max(tvmax, tv_workspace_bytes(items[i].B, items[i].H, items[i].W, K));
     off += r256(tvmax);
     L.total = off;
-    (void)energy_end;
     return L;
 }
+
+constexpr int kMinR = 8;  // least rows of a chunk
+constexpr size_t kWaitBytes = 3080;  // workspace of the wait selftest
 
 int check(const sci_batch_item *items, int n, int K) {
     SCI_CHECK_ARG(items && n >= 1 && n <= MAXI, "batch: 1..%d items (got %d)", MAXI, n);
@@ -261,10 +259,41 @@ int check(const sci_batch_item *items, int n, int K) {
     return SCI_OK;
 }
 
-int default_R(int64_t H, int64_t W, int64_t B) {
-    (void)W;
-    (void)B;
-    return H >= 1024 ? 256 : (H >= 256 ? 128 : 64);
+// Bands of one frame of the lean pass and the height of the chunks that R
+// rows at most make of it.
+int lean_bands(const sci_batch_item &s) {
+    return tv::band_count((int)s.W, s.cpl == 2 ? 64 : 128, 4, 4);
+}
+int even_R(int64_t H, int64_t R) {
+    const int64_t c = (H + R - 1) / R;
+    return (int)std::max<int64_t>(kMinR, (H + c - 1) / c);
+}
+
+// The least common chunk height (kMinR or more) at which the batch makes at
+// most `waves` times the work items that the GPU holds at a time: a pass
+// takes as long as its longest chain of rows, and a last wave that is nearly
+// empty as long as a full one.
+int waves_R(const sci_batch_item *items, int n, int waves) {
+    int64_t lo = kMinR, hi = kMinR;
+    for (int i = 0; i < n; ++i) hi = std::max(hi, items[i].H);
+    while (lo < hi) {
+        const int64_t R = (lo + hi) / 2;
+        int64_t c = 0;
+        for (int i = 0; i < n; ++i)
+            c += items[i].B * lean_bands(items[i]) * ((items[i].H + R - 1) / R);
+        if (c <= (int64_t)waves * resident_warps()) hi = R;
+        else lo = R + 1;
+    }
+    return (int)lo;
+}
+
+// For items without a chunk height: the fewest waves with chunks of at most
+// 96 rows (us per iteration by waves: see sci_batch_autotune).
+int default_R(const sci_batch_item *items, int n) {
+    int R = 0;
+    for (int w = 1; w <= 16; ++w)
+        if ((R = waves_R(items, n, w)) <= 96) break;
+    return R;
 }
 
 // Builds the host copy of the device table.
@@ -272,24 +301,34 @@ void build_table(const sci_batch_item *items, int n, int K, float eps, char *ws,
                  Table &T) {
     memset(&T, 0, sizeof(T));
     T.n = n;
+    const int R0 = default_R(items, n);
     T.proj_prefix[0] = T.tv_prefix[0] = T.qp_prefix[0] = T.tq_prefix[0] = 0;
+    // longest chunks first: the last wave's are short (16 / 64 items 10.15 /
+    // 82.2 ms in the caller's order, 10.05 / 81.5)
+    std::vector<int> ord(n);
+    for (int i = 0; i < n; ++i) ord[i] = i;
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+        return (items[a].R > 0 ? items[a].R : even_R(items[a].H, R0)) >
+               (items[b].R > 0 ? items[b].R : even_R(items[b].H, R0));
+    });
     for (int i = 0; i < n; ++i) {
-        const sci_batch_item &s = items[i];
+        const int k = ord[i];  // the item's place in the caller's list
+        const sci_batch_item &s = items[k];
         Item &I = T.it[i];
         I.y = s.y;
         I.bits = s.mask_bits;
         I.phisum = s.phisum;
         I.x = s.x;
-        I.xp = reinterpret_cast<float *>(ws + L.item_xp[i]);
-        I.y1 = reinterpret_cast<float *>(ws + L.item_y1[i]);
-        I.c = reinterpret_cast<float *>(ws + L.item_c[i]);
+        I.xp = reinterpret_cast<float *>(ws + L.item_xp[k]);
+        I.y1 = reinterpret_cast<float *>(ws + L.item_y1[k]);
+        I.c = reinterpret_cast<float *>(ws + L.item_c[k]);
         I.B = (int)s.B;
         I.hw = s.H * s.W;
         I.lam = s.lambda;
         tv::Pass &P = I.tv;
         P.f = I.xp;
         P.u = s.x;
-        P.energy = reinterpret_cast<double *>(ws + L.energy + L.item_e[i]);
+        P.energy = reinterpret_cast<double *>(ws + L.energy + L.item_e[k]);
         P.fs = I.hw;
         P.nf = (int)s.B;
         P.H = (int)s.H;
@@ -307,14 +346,14 @@ void build_table(const sci_batch_item *items, int n, int K, float eps, char *ws,
         P.own = 128 - 4 - 4;
         P.ht = K - 1;
         P.nbands = tv::band_count((int)s.W, 128, P.hl, P.hr);
-        P.R = s.R > 0 ? s.R : default_R(s.H, s.W, s.B);
+        P.R = s.R > 0 ? s.R : even_R(s.H, R0);
         P.nchunks = (int)((s.H + P.R - 1) / P.R);
         P.vec = 1;
         P.lag = 1;
         P.frame_fast = 1;
         T.proj_prefix[i + 1] = T.proj_prefix[i] + (int)((I.hw + PROJ_T - 1) / PROJ_T);
         T.qp_prefix[i + 1] = T.qp_prefix[i] + (int)((I.hw + QP_T - 1) / QP_T);
-        // the work-queue passes: the lean pipeline with the item's column
+        // the lean passes: the lean pipeline with the item's column
         // width, energies of even / odd iterations, stop decisions by ticket
         for (int par = 0; par < 2; ++par) {
             tv::Pass &Q = I.tvq[par];
@@ -329,9 +368,9 @@ void build_table(const sci_batch_item *items, int n, int K, float eps, char *ws,
             Q.own = 32 * cpl - 8;
             Q.nbands = tv::band_count((int)s.W, 32 * cpl, Q.hl, Q.hr);
             Q.energy = reinterpret_cast<double *>(ws + L.energy +
-                                                  (par ? L.item_e1[i] : L.item_e[i]));
-            Q.stopj = reinterpret_cast<int *>(ws + L.item_stop[i]);
-            Q.ticket = reinterpret_cast<unsigned *>(ws + L.item_stop[i] + sizeof(int) * s.B);
+                                                  (par ? L.item_e1[k] : L.item_e[k]));
+            Q.stopj = reinterpret_cast<int *>(ws + L.item_stop[k]);
+            Q.ticket = reinterpret_cast<unsigned *>(ws + L.item_stop[k] + sizeof(int) * s.B);
             // the fused iteration: the TV pass loads x_k and applies
             // x_k + lam (c phi_b) (the projection's rounding), writing x_{k+1}
             Q.f = par ? I.xp : I.x;
@@ -346,23 +385,9 @@ void build_table(const sci_batch_item *items, int n, int K, float eps, char *ws,
         T.tq_prefix[i + 1] =
             T.tq_prefix[i] + I.tvq[0].nbands * I.tvq[0].nchunks * I.tvq[0].nf;
     }
-    // (measured as fractions of n, 16 items / 64 items, ms: 1/16, 15/16 19.6 /
-    // 134; 0.25, 0.8 12.4 / 84.5; 0.3, 0.6 13.5 / 91.3; 0.4, 1 12.2 / 87.2;
-    // 0.5, 0.9 13.5 / 86.6; all phases of an iteration apart 12.8 / 93.0)
-    T.lag[PH_PROJ] = 0;
-    T.lag[PH_TV] = n < 2 ? 0 : std::max(1, n / 4);
-    T.lag[PH_FIX] = n < 2 ? 0 : std::max(T.lag[PH_TV], std::min(n - 1, 4 * n / 5));
-    T.order[0] = 0;
-    for (int s = 0; s < n; ++s)
-        for (int ph = 0; ph < 3; ++ph) {
-            const int i = (s + n - T.lag[ph]) % n;
-            T.order[3 * s + ph + 1] =
-                T.order[3 * s + ph] + (ph == PH_PROJ ? T.qp_prefix[i + 1] - T.qp_prefix[i]
-                                                     : T.tq_prefix[i + 1] - T.tq_prefix[i]);
-        }
 }
 
-// After an odd number of work-queue iterations the last x is in xp: copy
+// After an odd number of lean iterations the last x is in xp: copy
 // it into every item's x.
 __global__ void __launch_bounds__(PROJ_T) k_batch_copy_x(const Table *__restrict__ T) {
     const int g = blockIdx.x;
@@ -374,36 +399,39 @@ __global__ void __launch_bounds__(PROJ_T) k_batch_copy_x(const Table *__restrict
     for (int b = 0; b < I.B; ++b) I.x[b * I.hw + p] = I.xp[b * I.hw + p];
 }
 
-// bit 1 of the batch status: a bounded wait of a work-queue launch gave up
-__global__ void k_batch_fold(const Queue *Q) {
-    if (threadIdx.x == 0 && Q->abort) atomicOr(&g_batch_status, 2u);
+// A bounded wait of a grid that another one feeds, on purpose without one:
+// one warp polls a count that nothing raises at most `polls` times, then sets
+// bit 1 of the batch status.
+__global__ void k_wait_selftest(const unsigned *count, unsigned polls) {
+    unsigned ns = 32;
+    for (unsigned n = 0; n < polls; ++n) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+        if (v != 0u) return;
+        __nanosleep(ns);
+        if (ns < 1024) ns <<= 1;
+    }
+    if (threadIdx.x == 0) atomicOr(&g_batch_status, 2u);
 }
 
-// The give-up path of the work queue's bounded waits, on purpose: one warp
-// waits at most `polls` polls for a count that nothing raises, then raises
-// the abort flag, which the fold turns into status bit 1.
-__global__ void k_queue_wait_selftest(Queue *Q, unsigned polls) {
-    wait_count(Q, &Q->done[0][0], 1u, threadIdx.x & 31, polls);
-}
-
-int queue_selftest(unsigned polls, Queue *dQ, cudaStream_t s) {
-    SCI_CUDA(cudaMemsetAsync(dQ, 0, sizeof(Queue), s));
-    k_queue_wait_selftest<<<1, 32, 0, s>>>(dQ, polls);
-    SCI_LAUNCHED("k_queue_wait_selftest");
-    k_batch_fold<<<1, 32, 0, s>>>(dQ);
-    SCI_LAUNCHED("k_batch_fold");
+int wait_selftest(unsigned polls, unsigned *count, cudaStream_t s) {
+    SCI_CUDA(cudaMemsetAsync(count, 0, kWaitBytes, s));
+    k_wait_selftest<<<1, 32, 0, s>>>(count, polls);
+    SCI_LAUNCHED("k_wait_selftest");
     return SCI_OK;
 }
 
-// The work-queue form (sci_batch_queue.cu) unless SCI_BATCH_QUEUE=0.
-bool queue_enabled() {
+// The lean pass unless SCI_BATCH_QUEUE=0 or a mask is off the 16-byte
+// boundaries of its vector loads.
+bool lean_enabled(const Table &T) {
+    for (int i = 0; i < T.n; ++i)
+        if (reinterpret_cast<uintptr_t>(T.it[i].bits) & 15u) return false;
     const char *e = getenv("SCI_BATCH_QUEUE");
     return !(e && atoi(e) == 0);
 }
 
-// per_launch: iterations per persistent launch of the work queue (0: all).
 int enqueue(const Table &T, Table *dT, const Layout &L, char *ws, int n, int iters, int K,
-            int accelerate, int init_x0, int per_launch, cudaStream_t s) {
+            int accelerate, int init_x0, cudaStream_t s) {
     const int pb = T.proj_prefix[n], tb = (T.tv_prefix[n] + tv::WPB - 1) / tv::WPB;
     if (init_x0 || accelerate) {
         if (init_x0 && accelerate) k_batch_init<true, true><<<pb, PROJ_T, 0, s>>>(dT);
@@ -411,24 +439,16 @@ int enqueue(const Table &T, Table *dT, const Layout &L, char *ws, int n, int ite
         else k_batch_init<false, true><<<pb, PROJ_T, 0, s>>>(dT);
         SCI_LAUNCHED("k_batch_init");
     }
-    if (queue_enabled()) {
+    if (lean_enabled(T)) {
         // the items' stop decisions and tickets: a ticket counts the TV
         // tasks of an iteration and is reset by the last one, so it starts
         // at zero once per solve
-        SCI_CUDA(cudaMemsetAsync(ws + L.stop, 0, L.queue - L.stop, s));
-        Queue *dQ = reinterpret_cast<Queue *>(ws + L.queue);
-        const int m = per_launch > 0 ? per_launch : std::max(1, iters);
-        const int blocks = queue_blocks();
+        SCI_CUDA(cudaMemsetAsync(ws + L.stop, 0, L.tvscratch - L.stop, s));
         bool narrow = false;
-        for (int i = 0; i < n; ++i) narrow = narrow || T.it[i].tvq[0].cpl == 2;
-        for (int k0 = 0; k0 < iters; k0 += m) {
-            SCI_CUDA(cudaMemsetAsync(dQ, 0, sizeof(Queue), s));
-            if (int e = queue_launch(dT, dQ, k0, std::min(iters, k0 + m), accelerate != 0, K - 1,
-                                     blocks, narrow, s))
-                return e;
-            k_batch_fold<<<1, 32, 0, s>>>(dQ);
-            SCI_LAUNCHED("k_batch_fold");
-        }
+        for (int i = 0; i < n; ++i)
+            narrow = narrow || T.it[i].tvq[0].cpl == 2 || narrow_tail(T.it[i].tvq[0]);
+        for (int k = 0; k < iters; ++k)
+            if (int e = iteration_launch(T, dT, k, accelerate != 0, K - 1, narrow, s)) return e;
         if (iters & 1) {  // the last TV pass wrote xp
             k_batch_copy_x<<<pb, PROJ_T, 0, s>>>(dT);
             SCI_LAUNCHED("k_batch_copy_x");
@@ -469,7 +489,7 @@ int enqueue(const Table &T, Table *dT, const Layout &L, char *ws, int n, int ite
 // The whole solve of a batch (table upload, then the loop, captured once
 // into a cached CUDA graph when use_graph).
 int solve(const sci_batch_item *items, int n, int iters, int tv_iter_max, float eps,
-                 int accelerate, int init_x0, int use_graph, int per_launch, void *workspace,
+                 int accelerate, int init_x0, int use_graph, void *workspace,
                  size_t workspace_bytes, cudaStream_t s) {
     const Layout L = layout(items, n, tv_iter_max);
     SCI_CHECK_ARG(workspace && workspace_bytes >= L.total,
@@ -488,15 +508,14 @@ int solve(const sci_batch_item *items, int n, int iters, int tv_iter_max, float 
     }
     int rc = SCI_OK;
     if (!use_graph) {
-        rc = enqueue(*hT, dT, L, ws, n, iters, tv_iter_max, accelerate, init_x0, per_launch, s);
+        rc = enqueue(*hT, dT, L, ws, n, iters, tv_iter_max, accelerate, init_x0, s);
         delete hT;
         return rc;
     }
     std::string key(reinterpret_cast<const char *>(hT), sizeof(Table));
-    key_append(key, iters, accelerate, init_x0, per_launch);
+    key_append(key, iters, accelerate, init_x0);
     rc = run_graph("batch graph capture", key, s, [&](cudaStream_t cs) {
-        return enqueue(*hT, dT, L, ws, n, iters, tv_iter_max, accelerate, init_x0, per_launch,
-                       cs);
+        return enqueue(*hT, dT, L, ws, n, iters, tv_iter_max, accelerate, init_x0, cs);
     });
     delete hT;
     return rc;
@@ -527,91 +546,65 @@ int sci_batch_autotune(sci_batch_item *items, int n, int iters, int tv_iter_max,
     SCI_CHECK_ARG(iters >= 0, "batch: iters must be >= 0");
     cudaStream_t s = as_stream(stream);
     // Every candidate is timed on the batch itself -- a few iterations of its
-    // own solve from x0 = At(y / Phi_sum) (overwriting x), inside the
-    // persistent launch where all items share the GPU -- because a tiling
-    // timed on one item alone ranks differently there (measured on the
-    // 64-item uneven batch: per-shape single-item tuning 185 ms per solve,
-    // the default tiling 138 ms).  Candidates: row-chunk heights of
-    // 1/2, 1 and 2 times the default for each item's height (16..512 rows),
-    // 4 columns per lane for every item or 2 for items at most 256 columns
-    // wide; then, for the best tiling, 1, 2 or 3 iterations per launch
-    // against all of them.  The choice is cached per process for the batch's
-    // list of shapes.
+    // own solve from x0 = At(y / Phi_sum) (overwriting x): chunk heights that
+    // make 1, 2, 3 or 6 waves of work items of the TV pass.  Measured, us per
+    // iteration at 1 / 2 / 3 / 6: 4 items of up to 256 x 256 x 24 51 / 64 / 72;
+    // 6 of up to 512 x 512 x 32 185 / 186 / 193 / 230; 16 235 / 210 / 219 /
+    // 259; 64 of up to 1024 x 1024 x 32 1890 (1 to 3 waves are too few) / 1716.  The
+    // choice is cached per process for the batch's list of shapes.
     const int probe = std::max(1, std::min(iters, 6));
     std::string key;
     key_append(key, n, tv_iter_max, probe, accelerate);
     for (int i = 0; i < n; ++i) key_append(key, items[i].B, items[i].H, items[i].W);
     static std::mutex mu;
-    static std::map<std::string, std::tuple<int, int, int>> tuned;  // scale x 2, narrow, m
-    auto apply = [&](int scale2, int narrow) {
-        for (int i = 0; i < n; ++i) {
-            const int R = default_R(items[i].H, items[i].W, items[i].B) * scale2 / 2;
-            items[i].R = std::max(16, std::min(512, R));
-            items[i].cpl = (narrow && items[i].W <= 256) ? 2 : 4;
-        }
+    static std::map<std::string, int> tuned;  // chunk height
+    auto apply = [&](int R) {
+        for (int i = 0; i < n; ++i) items[i].R = even_R(items[i].H, R);
     };
+    for (int i = 0; i < n; ++i) items[i].cpl = 4;
+    if (iters_per_launch) *iters_per_launch = 0;
     {
         std::lock_guard<std::mutex> lk(mu);
         auto f = tuned.find(key);
         if (f != tuned.end()) {
-            apply(std::get<0>(f->second), std::get<1>(f->second));
-            if (iters_per_launch) *iters_per_launch = std::get<2>(f->second);
+            apply(f->second);
             return SCI_OK;
         }
     }
     cudaEvent_t e0, e1;
     SCI_CUDA(cudaEventCreate(&e0));
     SCI_CUDA(cudaEventCreate(&e1));
-    int rc = SCI_OK;
-    auto timed = [&](int m) -> float {  // the first run warms up
+    int rc = SCI_OK, bR = 0, last = 0;
+    float best = 1e30f;
+    for (int waves : {1, 2, 3, 6}) {
+        const int R = waves_R(items, n, waves);
+        if (R == last) continue;
+        last = R;
+        apply(R);
         float ms = 0.f;
-        for (int rep = 0; rep <= 2; ++rep) {
+        for (int rep = 0; rep <= 2 && rc == SCI_OK; ++rep) {  // the first run warms up
             cudaEventRecord(e0, s);
-            rc = solve(items, n, probe, tv_iter_max, eps, accelerate, 1, 0, m, workspace,
+            rc = solve(items, n, probe, tv_iter_max, eps, accelerate, 1, 0, workspace,
                        workspace_bytes, s);
-            if (rc != SCI_OK) return -1.f;
+            if (rc != SCI_OK) break;
             cudaEventRecord(e1, s);
             cudaEventSynchronize(e1);
             float t = 0.f;
             cudaEventElapsedTime(&t, e0, e1);
             if (rep > 0) ms += t;
         }
-        return ms;
-    };
-    float best = 1e30f;
-    int bs = 2, bn = 0, bm = 0;
-    for (int scale2 : {2, 1, 4}) {
-        for (int narrow : {0, 1}) {
-            apply(scale2, narrow);
-            const float ms = timed(0);
-            if (ms < 0.f) break;
-            if (ms < best) {
-                best = ms;
-                bs = scale2;
-                bn = narrow;
-            }
-        }
         if (rc != SCI_OK) break;
-    }
-    apply(bs, bn);
-    if (rc == SCI_OK && iters_per_launch) {
-        for (int m : {1, 2, 3}) {
-            if (m >= probe) continue;
-            const float ms = timed(m);
-            if (ms < 0.f) break;
-            if (ms < best) {
-                best = ms;
-                bm = m;
-            }
+        if (ms < best) {
+            best = ms;
+            bR = R;
         }
-        // a launch of all `probe` iterations stands for one of all iterations
-        *iters_per_launch = bm;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc == SCI_OK) {
+        apply(bR);
         std::lock_guard<std::mutex> lk(mu);
-        tuned[key] = std::make_tuple(bs, bn, bm);
+        tuned[key] = bR;
     }
     return rc;
 }
@@ -619,9 +612,9 @@ int sci_batch_autotune(sci_batch_item *items, int n, int iters, int tv_iter_max,
 int sci_batch_selftest_queue_wait(unsigned int polls, void *workspace, size_t workspace_bytes,
                                   void *stream) {
     SCI_CHECK_ARG(polls >= 1 && polls <= (1u << 20), "selftest: polls in [1, 2^20]");
-    SCI_CHECK_ARG(workspace && workspace_bytes >= sizeof(Queue),
-                  "selftest: a workspace of %zu bytes is needed", sizeof(Queue));
-    return queue_selftest(polls, static_cast<Queue *>(workspace), as_stream(stream));
+    SCI_CHECK_ARG(workspace && workspace_bytes >= kWaitBytes,
+                  "selftest: a workspace of %zu bytes is needed", kWaitBytes);
+    return wait_selftest(polls, static_cast<unsigned *>(workspace), as_stream(stream));
 }
 
 int sci_batch_gap_tv(const sci_batch_item *items, int n, int iters, int tv_iter_max, float eps,
@@ -630,8 +623,8 @@ int sci_batch_gap_tv(const sci_batch_item *items, int n, int iters, int tv_iter_
     if (int e = check(items, n, tv_iter_max)) return e;
     SCI_CHECK_ARG(iters >= 0, "batch: iters must be >= 0");
     SCI_CHECK_ARG(iters_per_launch >= 0, "batch: iters_per_launch must be >= 0");
-    return solve(items, n, iters, tv_iter_max, eps, accelerate, init_x0, use_graph,
-                 iters_per_launch, workspace, workspace_bytes, as_stream(stream));
+    return solve(items, n, iters, tv_iter_max, eps, accelerate, init_x0, use_graph, workspace,
+                 workspace_bytes, as_stream(stream));
 }
 
 }  // extern "C"

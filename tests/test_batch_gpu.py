@@ -173,3 +173,23 @@ def test_batch_config4_every_item_matches_single_solver():
         ref, _ = c_oracle.gap_tv(y, c_oracle.planar(mask), msum, x0, 50, 1.0, 0.1)
         r = np.linalg.norm(res[big].cpu().numpy() - ref) / np.linalg.norm(ref)
         assert r < 1e-4, r
+
+
+# Column bands of the lean launches at their edges: one band, a last band that
+# owns 4 to 60 columns (64 wide) and 64 (128 wide), chunks of 8 rows and of the
+# whole frame, against the generic launches.  The same arithmetic per pixel, so
+# the same bits.
+@pytest.mark.parametrize("W", [4, 128, 132, 184, 188, 248, 256, 304, 308])
+def test_lean_bands_equal_generic_launches(monkeypatch, W):
+    data = make_items([(37, W, 3, 0.5), (8, W, 32, 0.6), (70, W, 1, 0.5)], seed=W)
+    out = []
+    for env, R in (("0", 0), ("1", 0), ("1", 8), ("1", 70)):
+        monkeypatch.setenv("SCI_BATCH_QUEUE", env)
+        bs = sci.BatchSolver([d[2] for d in data], [d[1] for d in data], iters=5, tv_weight=0.1,
+                             eps=0.02, autotune=False)
+        for it in bs.items:
+            it.R = R
+        out.append([x.clone() for x in bs.run()])
+    for r in out[1:]:
+        for a, b in zip(out[0], r):
+            assert torch.equal(a, b)

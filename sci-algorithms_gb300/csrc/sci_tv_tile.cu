@@ -31,19 +31,25 @@ bool small(const Pass &P) { return Large::windows(P.nf, P.H, P.W) <= 300; }
 
 // Which calls run on tiles (slim: the lean row pipeline could run it, frames
 // of nf x H x W), by the number of windows.  A tile pass costs about 10 us +
-// 17 us per 1000 windows, halo and two barriers per update included; the row
-// pipelines have a chain of stages per row as their fixed part, about 24 us
-// (lean) and 28 us (generic), and less per pixel.  Measured, tile against
-// pipeline, us (windows):
-//   lean: 10 x 512 x 512 24.7 / 30.8 (1170), 16 x 512 x 512 32.9 / 37.1
-//   (1872), 4 x 1024 x 1024 34.9 / 35.0 (1976), 24 x 512 x 512 45.1 / 45.2
-//   (2808), 8 x 1024 x 1024 57 / 47 (3952), 24 x 2048 x 2048 560 / 310;
-//   generic: 10 x 517 x 643 31 / 45 (1560), 16 x 1001 x 1023 107 / 133
-//   (7600), 24 x 2045 x 2047 576 / 463 (45288); 30 steps (up to 8 passes): 10
-//   x 517 x 643 161 / 259, 16 x 1024 x 1024 602 / 792, 24 x 2048 x 2048 3130
-//   / 2570.
+// 11 to 13 us per 1000 windows, halo and two barriers per update included; the
+// row pipelines have a chain of stages per row as their fixed part, about 24
+// us (lean) and 28 us (generic), and less per pixel -- the lean one the less
+// the wider the frame, as its bands of 64 or 128 columns cover narrow frames
+// badly.  Measured, tile against pipeline, us (windows):
+//   lean, W <= 256: 64 x 256 x 256 32.2 / 37.4 (2240), 400 x 128 x 128 59.7 /
+//   60.9 (3600), 128 x 256 x 256 59.4 / 60.8 (4480), 256 x 256 x 256 120 / 100
+//   (8960); W <= 512: 20 x 384 x 384 25.3 / 33.9 (1400), 24 x 512 x 512 41.1 /
+//   45.2 (2808), 32 x 512 x 512 55.3 / 53.5 (3744); wider: 4 x 1024 x 1024
+//   31.0 / 34.4 (1976), 10 x 768 x 768 45.6 / 44.9 (2660, an iteration of a
+//   solve), 6 x 1024 x 1024 42.0 / 39.1 (2964), 24 x 2048 x 2048 560 / 310;
+//   generic: 10 x 517 x 643 31 / 45 (1560), 16 x 1001 x 1023 112 / 134
+//   (7600), 32 x 1001 x 1023 211 / 203 (15200), 24 x 2045 x 2047 604 / 467
+//   (45288); 30 steps (up to 8 passes): 10 x 517 x 643 161 / 259, 16 x 1024 x
+//   1024 617 / 795, 32 x 1024 x 1024 1144 / 1192 (15808), 12 x 2048 x 2048
+//   1614 / 1477.
 bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim) {
-    return Large::windows(nf, H, W) <= (slim ? 2000 : 14000);
+    const int64_t lean = W <= 256 ? 4500 : W <= 512 ? 3300 : 2500;
+    return Large::windows(nf, H, W) <= (slim ? lean : 14000);
 }
 
 void tile_geometry(Pass &P) {

@@ -26,6 +26,7 @@
 
 #include "sci_common.cuh"
 #include "sci_graph.cuh"
+#include "sci_sqerr.cuh"
 
 namespace sci {
 
@@ -148,16 +149,38 @@ __global__ void __launch_bounds__(256) k_proj_fwd(
     }
 }
 
-__global__ void k_mse(const float *__restrict__ a, const float *__restrict__ b,
-                      float *__restrict__ grad, float gscale, int64_t n, double *out) {
+// *out += sum (a - b)^2, or grad = gscale (a - b).  n4: groups of four with
+// 16-byte loads (0 where a pointer is not on such a boundary).  The squares in
+// float64 and scalar loads took 40 us at 16 x 256 x 256 x 8 (67 MB read).
+template <bool GRAD>
+__global__ void __launch_bounds__(256) k_mse(const float *__restrict__ a,
+                                             const float *__restrict__ b,
+                                             float *__restrict__ grad, float gscale, int64_t n,
+                                             int64_t n4, double *out) {
     double acc = 0.0;
-    GRID_LOOP(i, n) {
-        const float d = a[i] - b[i];
-        acc += (double)d * d;
-        if (grad) grad[i] = gscale * d;
+    SquareSum se;
+    se.clear();
+    int held = 0;
+    GRID_LOOP(q, n4) {
+        const float4 x = ldg4(a + 4 * q), y = ldg4(b + 4 * q);
+        if (GRAD) {
+            st4(grad + 4 * q, make_float4(gscale * (x.x - y.x), gscale * (x.y - y.y),
+                                          gscale * (x.z - y.z), gscale * (x.w - y.w)));
+        } else {
+            se.add4(x, y);
+            if (++held == 8) {
+                acc += se.take();
+                held = 0;
+            }
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && out) atomicAdd(out, acc);
+    GRID_LOOP(r, n - 4 * n4) {
+        const int64_t i = 4 * n4 + r;
+        const float d = a[i] - b[i];
+        if (GRAD) grad[i] = gscale * d;
+        else acc += (double)d * d;
+    }
+    if (!GRAD) rn_flush(acc + se.take(), out);
 }
 
 // --------------------------------------------------- projection adjoint
@@ -307,31 +330,77 @@ void launch_proj_bwd(int64_t hw, int N, cudaStream_t s, A... a) {
 }
 
 // Adjoint of x^0 = At(y / Phi_sum), y = A(x_true), Phi_sum = sum Phi_b and
-// Phi = sigmoid(logits): writes dlogits.
-__global__ void k_init_bwd(const float *__restrict__ x0b, const float *__restrict__ xt,
-                           const float *__restrict__ phi, const float *__restrict__ ps,
-                           const float *__restrict__ y, const float *__restrict__ ybar,
-                           float *__restrict__ phib, const float *__restrict__ psb,
-                           float *__restrict__ glog, float gscale, int N, int B, int64_t hw) {
-    GRID_LOOP(p, hw) {
-        const float s = ps[p];
-        float psacc = psb[p];
-        for (int n = 0; n < N; ++n) {
-            const int64_t i = (int64_t)n * hw + p;
-            const float *xbn = x0b + (int64_t)n * B * hw;
-            const float *xtn = xt + (int64_t)n * B * hw;
-            const float s0 = y[i] / s;
-            float s0b = 0.f;
-            for (int b = 0; b < B; ++b) s0b = fmaf(phi[b * hw + p], xbn[b * hw + p], s0b);
-            const float yt = ybar[i] + s0b / s;
-            psacc -= s0b * s0 / s;
-            for (int b = 0; b < B; ++b)
-                phib[b * hw + p] += fmaf(s0, xbn[b * hw + p], xtn[b * hw + p] * yt);
-        }
+// Phi = sigmoid(logits), in two passes: by item the adjoint of y (in place of
+// ybar) and of Phi_sum (t), by frame dPhi and with it dlogits.  As one pass
+// with a thread per pixel over items and frames, dPhi added up in memory, it
+// took 81 us at 16 x 256 x 256 x 8.
+template <int V>
+__global__ void __launch_bounds__(256) k_init_bwd_y(
+    const float *__restrict__ x0b, const float *__restrict__ phi, const float *__restrict__ ps,
+    const float *__restrict__ y, float *__restrict__ ybar, float *__restrict__ t, int N, int B,
+    int64_t hw) {
+    GRID_LOOP(g, (int64_t)N * hw / V) {
+        const int64_t i = g * V;
+        const int n = (int)(i / hw);
+        const int64_t p = i - (int64_t)n * hw;
+        const float *xn = x0b + (int64_t)n * B * hw + p;
+        float s0b[V], a[V], m[V], s[V], yb[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) s0b[e] = 0.f;
+#pragma unroll 8
         for (int b = 0; b < B; ++b) {
-            const float m = phi[b * hw + p];
-            glog[b * hw + p] = gscale * (phib[b * hw + p] + psacc) * m * (1.f - m);
+            ldv<V>(xn + b * hw, a);
+            ldv<V>(phi + b * hw + p, m);
+#pragma unroll
+            for (int e = 0; e < V; ++e) s0b[e] = fmaf(m[e], a[e], s0b[e]);
         }
+        ldv<V>(ps + p, s);
+        ldv<V>(y + i, a);
+        ldv<V>(ybar + i, yb);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            const float s0 = a[e] / s[e];
+            yb[e] = yb[e] + s0b[e] / s[e];
+            m[e] = s0b[e] * s0 / s[e];
+        }
+        stv<V>(ybar + i, yb);
+        stv<V>(t + i, m);
+    }
+}
+
+template <int V>
+__global__ void __launch_bounds__(256) k_init_bwd_phi(
+    const float *__restrict__ x0b, const float *__restrict__ xt, const float *__restrict__ phi,
+    const float *__restrict__ ps, const float *__restrict__ y, const float *__restrict__ ybar,
+    const float *__restrict__ t, const float *__restrict__ phib, const float *__restrict__ psb,
+    float *__restrict__ glog, int N, int B, int64_t hw) {
+    GRID_LOOP(g, (int64_t)B * hw / V) {
+        const int64_t i = g * V;
+        const int b = (int)(i / hw);
+        const int64_t p = i - (int64_t)b * hw;
+        float s[V], acc[V], sum[V];
+        ldv<V>(ps + p, s);
+        ldv<V>(psb + p, sum);
+        ldv<V>(phib + i, acc);
+#pragma unroll 4
+        for (int n = 0; n < N; ++n) {
+            float yn[V], yt[V], tn[V], xb[V], x[V];
+            ldv<V>(y + n * hw + p, yn);
+            ldv<V>(ybar + n * hw + p, yt);
+            ldv<V>(t + n * hw + p, tn);
+            ldv<V>(x0b + ((int64_t)n * B + b) * hw + p, xb);
+            ldv<V>(xt + ((int64_t)n * B + b) * hw + p, x);
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+                sum[e] -= tn[e];
+                acc[e] += fmaf(yn[e] / s[e], xb[e], x[e] * yt[e]);
+            }
+        }
+        float m[V];
+        ldv<V>(phi + i, m);
+#pragma unroll
+        for (int e = 0; e < V; ++e) m[e] = (acc[e] + sum[e]) * m[e] * (1.f - m[e]);
+        stv<V>(glog + i, m);
     }
 }
 
@@ -447,7 +516,10 @@ int forward(const float *logits, const float *lambdas, const float *xt, int64_t 
         if (e) return e;
     }
     SCI_CUDA(cudaMemsetAsync(w.loss, 0, sizeof(double), s));
-    k_mse<<<grid1(nbhw, 256), 256, 0, s>>>(w.X + K * nbhw, xt, nullptr, 0.f, nbhw, w.loss);
+    const float *XK = w.X + K * nbhw;
+    const int64_t n4 = aligned16(XK) && aligned16(xt) ? nbhw / 4 : 0;
+    k_mse<false><<<std::min(4u * kSMs, grid1(n4 ? n4 : nbhw, 256).x), 256, 0, s>>>(
+        XK, xt, nullptr, 0.f, nbhw, n4, w.loss);
     SCI_LAUNCHED("k_mse");
     return SCI_OK;
 }
@@ -527,10 +599,11 @@ int sci_unrolled_bwd(const float *logits, const float *lambdas, const float *x_t
     // workspace (same arguments) are used as they are.
     const int64_t hw = H * W, nbhw = N * B * hw, nhw = N * hw, nf = N * B;
     const int T = tv_iters, U = T - 1;
-    const dim3 g = grid1(nbhw, 256), gp = grid1(hw, 128);
     // dL/dx^K = grad_loss * 2 (x^K - x_true) / numel
-    k_mse<<<g, 256, 0, s>>>(w.X + (int64_t)K * nbhw, x_true, w.xb,
-                            2.f * grad_loss / (float)nbhw, nbhw, nullptr);
+    const float *XK = w.X + (int64_t)K * nbhw;
+    const int64_t n4 = aligned16(XK) && aligned16(x_true) && aligned16(w.xb) ? nbhw / 4 : 0;
+    k_mse<true><<<grid1(n4 ? n4 : nbhw, 256), 256, 0, s>>>(
+        XK, x_true, w.xb, 2.f * grad_loss / (float)nbhw, nbhw, n4, nullptr);
     SCI_LAUNCHED("k_mse");
     SCI_CUDA(cudaMemsetAsync(w.y1c, 0, 4 * nhw, s));
     SCI_CUDA(cudaMemsetAsync(w.ybar, 0, 4 * nhw, s));
@@ -565,8 +638,20 @@ int sci_unrolled_bwd(const float *logits, const float *lambdas, const float *x_t
                                w.phib, w.psb, grad_lambdas, w.xb, (int)N, (int)B, hw);
         SCI_LAUNCHED("k_proj_bwd");
     }
-    k_init_bwd<<<gp, 128, 0, s>>>(w.xb, x_true, w.phi, w.ps, w.y, w.ybar, w.phib, w.psb,
-                                  grad_logits, 1.f, (int)N, (int)B, hw);
+    // y1c is the last of the carries that the loop used: scratch from here on
+    if (v4 && aligned16(x_true) && aligned16(grad_logits)) {
+        k_init_bwd_y<4><<<grid1(nhw / 4, 256), 256, 0, s>>>(w.xb, w.phi, w.ps, w.y, w.ybar, w.y1c,
+                                                            (int)N, (int)B, hw);
+        k_init_bwd_phi<4><<<grid1(B * hw / 4, 256), 256, 0, s>>>(
+            w.xb, x_true, w.phi, w.ps, w.y, w.ybar, w.y1c, w.phib, w.psb, grad_logits, (int)N,
+            (int)B, hw);
+    } else {
+        k_init_bwd_y<1><<<grid1(nhw, 256), 256, 0, s>>>(w.xb, w.phi, w.ps, w.y, w.ybar, w.y1c,
+                                                        (int)N, (int)B, hw);
+        k_init_bwd_phi<1><<<grid1(B * hw, 256), 256, 0, s>>>(
+            w.xb, x_true, w.phi, w.ps, w.y, w.ybar, w.y1c, w.phib, w.psb, grad_logits, (int)N,
+            (int)B, hw);
+    }
     SCI_LAUNCHED("k_init_bwd");
     return SCI_OK;
     });

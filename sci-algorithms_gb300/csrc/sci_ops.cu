@@ -361,7 +361,8 @@ static void launch_admm_smem(const float *th, const float *bb, Mask<MODE> M, con
 // TV kernel while it loads x (same arithmetic as k_proj_gap).
 // SQ: also adds sum (orig - x)^2 to *sq, the squared error of the iteration
 // that produced x.  In a pass of its own that read x once more and was a
-// launch: 4.8 of the 21 us of a 256 x 256 x 8 iteration; fused, 16.5 us.
+// launch: 15.8 us an iteration at 256 x 256 x 8 and 585 at 2048 x 2048 x 24
+// against 14.9 and 501 (12.2 and 416 without a ground truth).
 template <int MODE, bool ACC, bool SQ>
 __global__ void __launch_bounds__(256) k_gap_resid_vec(
     const float *__restrict__ x, Mask<MODE> M, const float *__restrict__ y,
@@ -426,7 +427,9 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
 // pass reads t (t = theta_0 + 0 at the first iteration), forms
 // yb = sum_b phi_b t_b and r_{k+1} = (y - yb) / (phisum + gamma).  With xo
 // it also writes x = t + lambda (r phi_b) of every frame (a second sweep).
-// SQ (with WANT_X): also adds sum (orig - x)^2 to *sq.
+// SQ: also adds sum (orig - x)^2 to *sq, x stored or not (2048 x 2048 x 24: an
+// iteration 698 us with x stored for a pass of its own, 603 with it stored
+// here, 551 without).
 template <bool FIRST, bool WANT_X, bool SQ>
 __global__ void __launch_bounds__(256) k_admm_resid_vec(
     const float *__restrict__ tp, Mask<1> M, const float *__restrict__ y,
@@ -466,7 +469,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
                                      __fdiv_rn(yv.w - s.w, ps.w + gamma));
         if (rn) rn_add4(racc, r);
         st4(rnew + p, r);
-        if (WANT_X) {
+        if (WANT_X || SQ) {
 #pragma unroll 4
             for (int b = 0; b < B; ++b) {
                 const float4 m = M.at4(b, p, w);
@@ -474,7 +477,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
                 const float4 xv =
                     make_float4(fmaf(lam, r.x * m.x, t.x), fmaf(lam, r.y * m.y, t.y),
                                 fmaf(lam, r.z * m.z, t.z), fmaf(lam, r.w * m.w, t.w));
-                st4(xo + b * hw + p, xv);
+                if (WANT_X) st4(xo + b * hw + p, xv);
                 if (SQ) se.add4(ldg4(orig + b * hw + p), xv);
                 if (SQ && (b & 7) == 7) sacc += se.take();
             }
@@ -745,17 +748,19 @@ int admm_residual_rn(const float *t, const uint32_t *mask_bits, const float *y,
     const int T = resid_threads(hw);
     const dim3 g = grid_for(hw / 4, T);
     Mask<1> M{mask_bits, hw};
-    // x is written, and its squared error summed, by the same kernel
-    const bool fuse = sq && x_out && orig && aligned16(orig);
+    const bool fuse = sq && orig && aligned16(orig);
+    SCI_CHECK_ARG(fuse || !sq || x_out, "sci_admm_residual: the squared error needs x_out");
 #define SCI_ADMM_RESID(F, X, Q)                                                              \
     SCI_CUDA(launch_dep(k_admm_resid_vec<F, X, Q>, g, dim3(T), 0, s, t, M, y, phisum, r_new, \
                         x_out, lambda, gamma, (int)B, hw, rn, zero, nzero, resid_rev(), orig, sq))
     if (first) {
-        if (fuse) SCI_ADMM_RESID(true, true, true);
+        if (fuse && x_out) SCI_ADMM_RESID(true, true, true);
+        else if (fuse) SCI_ADMM_RESID(true, false, true);
         else if (x_out) SCI_ADMM_RESID(true, true, false);
         else SCI_ADMM_RESID(true, false, false);
     } else {
-        if (fuse) SCI_ADMM_RESID(false, true, true);
+        if (fuse && x_out) SCI_ADMM_RESID(false, true, true);
+        else if (fuse) SCI_ADMM_RESID(false, false, true);
         else if (x_out) SCI_ADMM_RESID(false, true, false);
         else SCI_ADMM_RESID(false, false, false);
     }

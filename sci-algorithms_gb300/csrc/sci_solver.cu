@@ -261,7 +261,10 @@ int enqueue(const Args &a, cudaStream_t s) {
         int nzero = 0;
         double *zero = tv_clear_region(B, H, W, K, w.tv, &nzero);
         for (int it = 0; it < o.iters; ++it) {
-            const bool want_x = (it == o.iters - 1) || (o.orig && o.sqerr);
+            // x: the result, and for the squared error where the residual
+            // pass cannot add it up (as it decides)
+            const bool want_x =
+                it == o.iters - 1 || (o.orig && o.sqerr && !aligned16(o.orig));
             const float gamma = o.gammas ? o.gammas[it] : o.gamma;
             float *cur = T[it & 1], *nxt = T[(it + 1) & 1];
             int e = admm_residual_rn(it ? tb : cur, a.bits, a.y, a.phisum, R,

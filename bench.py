@@ -742,7 +742,7 @@ def run_kernel(args):
 def run_batch(args):
     """Profiling mode for the batched solve: ``--launches`` solves of the
     first ``--frames`` items of the 64-item uneven batch (50 iterations,
-    autotuned), the loop replayed from its CUDA graph."""
+    autotuned), launched without a CUDA graph."""
     import torch
     import sci_algorithms_gb300 as sci
     meas, masks, elems = [], [], 0

@@ -305,9 +305,10 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
     SCI_CHECK_ARG(!ra.tout || (proj && slim), "tv: the t output needs the lean pass with the "
                                               "on-load projection (aligned frames)");
     const int pmode = !proj ? 0 : ra.detector ? 5 : ra.tout ? 3 : ra.phi ? 2 : 1;  // the lean pass's PROJ
-    // the clip rule in one pass on the lean pipeline (4 columns per lane)
+    // the clip rule in one pass on the lean pipeline (4 columns per lane), with
+    // any row chunking: tvx_proj_supported answers for it
     const bool clip = slim_enabled() && ra.rule == RULE_CLIP && !resid && U <= SMAX &&
-                      force_R <= 0 && !getenv("SCI_TV_R") && aligned_for(4);
+                      aligned_for(4);
     SCI_CHECK_ARG(!ra.detector || use_tiles(nf, H, W, slim),
                   "tv: the spectral on-load projection needs tiles");
     SCI_CHECK_ARG(!proj || ra.detector || slim || clip || !(ra.phi || ra.rule == RULE_CLIP),

@@ -388,3 +388,32 @@ def test_squared_error_of_the_residual_passes(H, W, B, kind, gray):
         sums.append(s.sqerr.cpu().numpy()[:4].copy())
     assert np.all(sums[0] > 0)
     np.testing.assert_allclose(sums[0], sums[1], rtol=1e-12)
+
+
+def same(a, b):
+    """Equal values, NaN where the other is NaN."""
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a),
+                                                                      torch.nan_to_num(b))
+
+
+# Every switch that shapes the TV pass leaves a solve's values alone, whatever
+# the mask and the denoiser (their passes perform the same operations).
+@pytest.mark.parametrize("switch", ["SCI_TV_R=8", "SCI_TV_R=64", "SCI_TV_LAG=2", "SCI_TV_CPL=2",
+                                    "SCI_TV_CPL=4", "SCI_TV_ORDER=0", "SCI_SLIM_MINB=3",
+                                    "SCI_TV_FORM=0", "SCI_TV_SLIM=0", "SCI_TV_TILE=0",
+                                    "SCI_TV_TILE=1", "SCI_FUSED_PROJ=0"])
+@pytest.mark.parametrize("gray", [True, False])
+@pytest.mark.parametrize("tvm", ["tv_chambolle", "ATV_ClipA", "ATV_ClipB"])
+def test_gap_solve_under_every_tv_switch(monkeypatch, switch, gray, tvm):
+    H, W, B = 100, 260, 4
+    g = torch.Generator(device="cuda").manual_seed(7)
+    mask = torch.rand(H, W, B, device="cuda", generator=g)
+    if not gray:
+        mask = (mask < 0.5).float()
+    op = sci.MaskOperator(mask)
+    y = op.phi.sum(0) * torch.rand(H, W, device="cuda", generator=g)
+    out = []
+    for name, value in (("SCI_PDL", "1"), switch.split("=")):
+        monkeypatch.setenv(name, value)
+        out.append(sci.Solver(op, "gap", 4, 0.9, 0.1, 5, tvm=tvm, eps=0.0).run(y).clone())
+    assert torch.equal(*out)

@@ -178,10 +178,12 @@ int enqueue(const Args &a, cudaStream_t s) {
     // FP64 ||r||^2 of iteration `it`'s projection residual (nullable)
     auto rn = [&](int it) { return o.resid_norm ? o.resid_norm + it : nullptr; };
     auto sq = [&](int it) { return o.sqerr ? o.sqerr + it : nullptr; };
-    const bool aligned = ((reinterpret_cast<uintptr_t>(a.x0) | reinterpret_cast<uintptr_t>(a.x_out) |
-                           reinterpret_cast<uintptr_t>(a.y) | reinterpret_cast<uintptr_t>(a.phisum) |
-                           reinterpret_cast<uintptr_t>(a.bits) | (a.bits ? 0 : reinterpret_cast<uintptr_t>(a.phi))) & 15u) == 0;
     const bool packed = a.bits != nullptr;
+    // for the fused iterations' 16-byte loads (the workspace holds y1, the
+    // residual map and stacks)
+    const bool aligned = aligned16(a.x0) && aligned16(a.x_out) && aligned16(a.y) &&
+                         aligned16(a.phisum) && aligned16(a.ws) &&
+                         (packed ? aligned16(a.bits) : aligned16(a.phi));
     if (!a.admm && aligned && hw % 4 == 0 &&
         (o.tvm ? tvx_proj_supported(o.tvm, B, W, K, packed) : tv_proj_supported(B, W, K, packed))) {
         // Fused iteration: a read-only pass forms the residual map c (and

@@ -417,3 +417,22 @@ def test_gap_solve_under_every_tv_switch(monkeypatch, switch, gray, tvm):
         monkeypatch.setenv(name, value)
         out.append(sci.Solver(op, "gap", 4, 0.9, 0.1, 5, tvm=tvm, eps=0.0).run(y).clone())
     assert torch.equal(*out)
+
+
+# A workspace on an 8-byte boundary (its float64 sums need no more): the fused
+# iteration's vector loads of it do not apply, the projection kernels' do.
+@pytest.mark.parametrize("gray,tvm", [(True, "tv_chambolle"), (True, "ATV_ClipA"),
+                                      (False, "ATV_ClipA"), (True, "ITV2D_FGP")])
+def test_workspace_on_an_8_byte_boundary(gray, tvm):
+    H, W, B = 40, 132, 3
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mask = torch.rand(H, W, B, device="cuda", generator=g)
+    if not gray:
+        mask = (mask < 0.5).float()
+    op = sci.MaskOperator(mask)
+    y = op.phi.sum(0) * torch.rand(H, W, device="cuda", generator=g)
+    s = sci.Solver(op, "gap", 4, 0.9, 0.1, 5, tvm=tvm, eps=0.0)
+    ref = s.run(y).clone()
+    n = s.ws.numel()
+    s.ws = torch.empty(n + 16, dtype=torch.uint8, device="cuda")[8:8 + n]
+    assert torch.equal(s.run(y), ref)

@@ -173,9 +173,15 @@ __device__ __forceinline__ void fetch(const Pass &P, const Rings &G, const float
     cp_commit();
 }
 
+// proj_px with the product formed: where c is not finite, frames whose bit is
+// not set get fmaf(lam, c * 0, x), as the projection kernels give them.
+__device__ __forceinline__ float proj_mul(float lam, float c, float x, uint32_t w, uint32_t fbit) {
+    return fmaf(lam, c * ((w & fbit) ? 1.f : 0.f), x);
+}
+
 // Stage 0 of step r: u_0 = f at row r from the input ring (with PROJ the
 // projection applied, and f written back for the later stages).
-template <int CPL, int PROJ>
+template <int CPL, int PROJ, int FORM>
 __device__ __forceinline__ Row<CPL> stage0(const Pass &P, const Rings &G, int r, int frame) {
     constexpr int NQ = Geo<CPL>::NQ;
     Row<CPL> u = lds<CPL>(G.x, r);
@@ -185,9 +191,14 @@ __device__ __forceinline__ Row<CPL> stage0(const Pass &P, const Rings &G, int r,
         const uint32_t fbit = 1u << frame;
 #pragma unroll
         for (int j = 0; j < NQ; ++j)
-            if (PROJ == 2) u.q[j] = fma2(mk2(P.lam, P.lam), mul2(c.q[j], wb.q[j]), u.q[j]);
-            else u.q[j] = mk2(proj_px(P.lam, lo(c.q[j]), lo(u.q[j]), __float_as_uint(lo(wb.q[j])), fbit),
-                         proj_px(P.lam, hi(c.q[j]), hi(u.q[j]), __float_as_uint(hi(wb.q[j])), fbit));
+            if (PROJ == 2)
+                u.q[j] = fma2(mk2(P.lam, P.lam), mul2(c.q[j], wb.q[j]), u.q[j]);
+            else if (FORM == 2)
+                u.q[j] = mk2(proj_mul(P.lam, lo(c.q[j]), lo(u.q[j]), __float_as_uint(lo(wb.q[j])), fbit),
+                             proj_mul(P.lam, hi(c.q[j]), hi(u.q[j]), __float_as_uint(hi(wb.q[j])), fbit));
+            else
+                u.q[j] = mk2(proj_px(P.lam, lo(c.q[j]), lo(u.q[j]), __float_as_uint(lo(wb.q[j])), fbit),
+                             proj_px(P.lam, hi(c.q[j]), hi(u.q[j]), __float_as_uint(hi(wb.q[j])), fbit));
         sts<CPL>(G.x, r, u);
     }
     return u;
@@ -325,7 +336,7 @@ __device__ __forceinline__ void sstep(const Pass &P, const SS<S, CPL> &in, SS<S,
     fetch<CPL, PROJ, COH>(P, G, fb, r + PF, min(r + PF, P.H - 1), L.colc, ldb, frame);
     cp_wait<PF>();
     if (COH && CPL == 2) __syncwarp();  // the pair's copy was the even lane's
-    Row<CPL> ucur = (!GEN || r < P.H) ? stage0<CPL, PROJ>(P, G, r, frame) : zrow<CPL>();
+    Row<CPL> ucur = (!GEN || r < P.H) ? stage0<CPL, PROJ, FORM>(P, G, r, frame) : zrow<CPL>();
     stages<S, 1, CPL, ENERGY, MODE, GEN, FORM, PROJ == 3>(P, in, out, ucur, r, rs, r0, r1, L, ob, G,
                                                         ek);
 }

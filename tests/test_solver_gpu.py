@@ -436,3 +436,33 @@ def test_workspace_on_an_8_byte_boundary(gray, tvm):
     n = s.ws.numel()
     s.ws = torch.empty(n + 16, dtype=torch.uint8, device="cuda")[8:8 + n]
     assert torch.equal(s.run(y), ref)
+
+
+# A dead or saturated pixel of the measurement: the projection on load of
+# float masks and of the clip denoisers gives the values of the projection
+# kernel, x + lambda (c phi), also where c is not finite and phi is 0.
+@pytest.mark.parametrize("gray,tvm", [(True, "tv_chambolle"), (True, "ATV_ClipA"),
+                                      (False, "ATV_ClipA"), (False, "ATV_ClipB")])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("W", [96, 260])
+def test_bad_measurement_pixel_on_the_fused_path(monkeypatch, gray, tvm, bad, W):
+    H, B = 60, 4
+    g = torch.Generator(device="cuda").manual_seed(5)
+    mask = torch.rand(H, W, B, device="cuda", generator=g)
+    if not gray:
+        mask = (mask < 0.5).float()
+    op = sci.MaskOperator(mask)
+    y = op.phi.sum(0) * torch.rand(H, W, device="cuda", generator=g)
+    y[20, 70] = bad
+    y[H - 1, W - 1] = bad
+    x0 = torch.rand(B, H, W, device="cuda", generator=g)
+    out = []
+    for fused, tile in (("0", "0"), ("1", "0"), ("1", "1")):
+        monkeypatch.setenv("SCI_FUSED_PROJ", fused)
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        for iters in (1, 2):
+            out.append(sci.Solver(op, "gap", iters, 0.9, 0.1, 5, tvm=tvm, eps=0.0).run(
+                y, x0=x0.clone()).clone())
+    assert not torch.isfinite(out[0]).all()
+    for i in range(2, 6):
+        assert same(out[i % 2], out[i])

@@ -59,11 +59,43 @@ struct Metrics {
     double *sqerr, *ssim_sum;
     int H, W, rows, nbands, nchunks;
     int64_t items;
-    float scale;         // power of two near 1 / data_range: exact
-    double unscale2;     // 1 / scale^2
+    float scale;         // power of two near 1 / data_range, for the windows
     // 49^2 C1 and 7 48 C2 of the scaled frames, as pairs
     float c1, c1_lo, c2, c2_lo;
+    double C1, C2;       // of the frames as they are
 };
+
+// 1 - SSIM of the window around (i, j), its moments about the means as float32
+// sums over the window and the quotient in float64, of the frames as they are:
+// for windows whose squared sums the packed form cannot hold (frames far
+// outside the data range) and those with a value that is not a number.
+__device__ __forceinline__ double wide_window(const float *a, const float *b, int W, int i, int j,
+                                              double C1, double C2) {
+    float sx = 0.f, sy = 0.f, vx = 0.f, vy = 0.f, vxy = 0.f, mx = 0.f, my = 0.f;
+#pragma unroll 1
+    for (int t = 0; t < 2 * WIN; ++t) {
+        const int64_t p = (int64_t)(i - R + (t < WIN ? t : t - WIN)) * W + (j - R);
+        if (t == WIN) {
+            mx = sx * (1.f / (WIN * WIN));
+            my = sy * (1.f / (WIN * WIN));
+        }
+#pragma unroll 1
+        for (int v = 0; v < WIN; ++v) {
+            const float x = a[p + v], y = b[p + v], dx = x - mx, dy = y - my;
+            if (t < WIN) {
+                sx += x;
+                sy += y;
+            } else {
+                vx = fmaf(dx, dx, vx);
+                vy = fmaf(dy, dy, vy);
+                vxy = fmaf(dx, dy, vxy);
+            }
+        }
+    }
+    const double n = 1.0 / (WIN * WIN - 1), Mx = mx, My = my;
+    return 1.0 - ((2.0 * Mx * My + C1) * (2.0 * (n * vxy) + C2)) /
+                     ((Mx * Mx + My * My + C1) * (n * vx + n * vy + C2));
+}
 
 // v / (h + c + c_lo).  The rounding of h + c goes into the reciprocal's
 // Newton step: left out, it has one sign for whole binades of h (c's last
@@ -133,20 +165,24 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
     Comp ds = {0.f, 0.f};
     double sse = 0.0, dssim = 0.0;
 
-    // A new row: its (s, d) into slot q, its squared error into the sums.
+    // A new row: its (s, d), scaled, into slot q, its squared error into the
+    // sums (as it is: SquareSum holds any range, and a scaled value could
+    // leave float32's).
     auto take_row = [&](float4 va, float4 vb, f2 (&q)[4], bool count) {
-        const float x[4] = {va.x * P.scale, va.y * P.scale, va.z * P.scale, va.w * P.scale};
-        const float y[4] = {vb.x * P.scale, vb.y * P.scale, vb.z * P.scale, vb.w * P.scale};
+        const float x[4] = {va.x, va.y, va.z, va.w}, y[4] = {vb.x, vb.y, vb.z, vb.w};
+        float d[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = mk2(x[k] + y[k], x[k] - y[k]);
-        if (count) {
-            const float d[4] = {hi(q[0]), hi(q[1]), hi(q[2]), hi(q[3])};
-            se.add4(x, y, d);
+        for (int k = 0; k < 4; ++k) {
+            d[k] = x[k] - y[k];
+            q[k] = mk2((x[k] + y[k]) * P.scale, d[k] * P.scale);
         }
+        if (count) se.add4(x, y, d);
     };
     // The windows of one row of centres, from the sums of the common six
-    // rows and the seventh row `o`; held rows are p[1 .. 6] and o.
+    // rows and the seventh row `o`; held rows are p[1 .. 6] and o.  Returns
+    // the windows left to wide_window, a bit each.
     auto windows = [&](const f2 (&common)[4], const f2 (&o)[4]) {
+        unsigned wide = 0u;
         f2 T[10], M[10];  // columns col - 3 .. col + 6: sum and centred sum of squares
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -190,10 +226,14 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
             // over 7 48, so that no factor is rounded
             V = fma2(V, seven, w);
             const f2 S2 = mul2(S, S);
-            const float e1 = quotient(hi(S2), 0.5f * (lo(S2) + hi(S2)), P.c1, P.c1_lo);
-            const float e2 = quotient(hi(V), 0.5f * (lo(V) + hi(V)), P.c2, P.c2_lo);
-            ds.add(fmaf(-e1, e2, e1 + e2) * win[k], 0.f);
+            const float h1 = 0.5f * (lo(S2) + hi(S2)), h2 = 0.5f * (lo(V) + hi(V));
+            const float e1 = quotient(hi(S2), h1, P.c1, P.c1_lo);
+            const float e2 = quotient(hi(V), h2, P.c2, P.c2_lo);
+            const bool held = h1 + h2 < 1e30f;
+            ds.add(held ? fmaf(-e1, e2, e1 + e2) * win[k] : 0.f, 0.f);
+            if (!held && win[k] != 0.f) wide |= 1u << k;
         }
+        return wide;
     };
 
     float4 n0a = load4<VEC>(pa + (int64_t)q0 * W, col, W);
@@ -218,8 +258,9 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
             common[k] = add2(add2(add2(p[1][k], p[2][k]), add2(p[3][k], p[4][k])),
                              add2(p[5][k], p[6][k]));
         const int i = row - R;  // centre of rows row - 6 .. row
-        if (i >= i0 && i < i1) windows(common, p[0]);
-        if (i + 1 >= i0 && i + 1 < i1) windows(common, p[7]);
+        unsigned wide = 0u;
+        if (i >= i0 && i < i1) wide = windows(common, p[0]);
+        if (i + 1 >= i0 && i + 1 < i1) wide |= windows(common, p[7]) << 4;
         if ((row & 6) == 6) {
             const double a = se.take();
             sse += own ? a : 0.0;
@@ -229,12 +270,16 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
         for (int r = 0; r < WIN - 1; ++r)
 #pragma unroll
             for (int k = 0; k < 4; ++k) p[r][k] = p[r + 2][k];
+        for (; wide; wide &= wide - 1) {
+            const int t = __ffs(wide) - 1;
+            dssim += wide_window(pa, pb, W, i + (t >> 2), col + (t & 3), P.C1, P.C2);
+        }
+        __syncwarp();
     }
     const double a = se.take();
     sse += own ? a : 0.0;
     dssim += ds.take();
     double ss = wins ? (double)wins * max(0, i1 - i0) - dssim : 0.0;
-    sse *= P.unscale2;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         sse += __shfl_xor_sync(0xffffffffu, sse, o);
@@ -272,9 +317,10 @@ extern "C" int sci_frame_metrics(const float *orig, const float *x, int64_t nfra
     // frames scaled by a power of two to a data range in [1, 2)
     const int e = std::max(-120, std::min(120, ilogb(data_range)));
     P.scale = (float)ldexp(1.0, -e);
-    P.unscale2 = ldexp(1.0, 2 * e);
-    const double c1 = 2401.0 * (0.01 * data_range) * (0.01 * data_range) / P.unscale2;
-    const double c2 = 336.0 * (0.03 * data_range) * (0.03 * data_range) / P.unscale2;
+    P.C1 = (0.01 * data_range) * (0.01 * data_range);
+    P.C2 = (0.03 * data_range) * (0.03 * data_range);
+    const double unscale2 = ldexp(1.0, 2 * e);
+    const double c1 = 2401.0 * P.C1 / unscale2, c2 = 336.0 * P.C2 / unscale2;
     P.c1 = (float)c1;
     P.c1_lo = (float)(c1 - P.c1);
     P.c2 = (float)c2;

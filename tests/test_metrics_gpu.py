@@ -103,3 +103,28 @@ def test_frame_metrics_bad_pixel_stays_in_its_frame(bad):
     assert np.isfinite([se[0], se[2], ss[0], ss[2]]).all()
     keep = [0, 2]
     _check(a[keep].contiguous(), b[keep].contiguous())
+
+
+# Frames far outside [0, data_range]: window means and moments are float32 of
+# the frames as they are (finite up to 1e18 and more), quotients and squared
+# errors do not depend on the range.  The tolerance is _check's, with the
+# denominators' 1 - SSIM up to 2.
+@pytest.mark.parametrize("size,data_range", [(1e18, 1.0), (1.0, 1e-18), (1e17, 0.25),
+                                             (1e10, 1e-12), (1e-18, 1e18), (1e-3, 1e37),
+                                             (1e18, 1e36), (1e-30, 1e-36)])
+def test_frame_metrics_far_outside_the_data_range(size, data_range):
+    a, b = _pair(2, 41, 150, noise=0.2)
+    _check(a * size, b * size, data_range)
+    # one frame of the stack, one window of the frame
+    c, d = a.clone(), b.clone()
+    c[1] *= size
+    d[1] *= size
+    _check(c, d, data_range)
+
+
+def test_frame_psnr_of_values_near_the_float32_limit():
+    a, b = _pair(1, 20, 30)
+    for size, data_range in ((3e38, 1e-12), (1e30, 1e-25), (1e-37, 1.0), (1e-30, 1e38)):
+        psnr, _ = frame_psnr_ssim(a * size, b * size, data_range)
+        na, nb = ((t * size).cpu().numpy()[0].astype(np.float64) for t in (a, b))
+        assert abs(psnr[0] - port.compare_psnr(na, nb, data_range=data_range)) < 1e-11

@@ -22,8 +22,7 @@
 //    them shuffled in per lane of 4).
 //  * Moments are merged, not subtracted: sum (p - m)^2 of a column about its
 //    own mean, then sum over columns of those plus the spread of the column
-//    means.  No cancellation, so float32 keeps the accuracy of the direct
-//    two-pass sums.
+//    means.  No cancellation.
 //  * The two moments needed are those of s = x + y and d = x - y, carried as
 //    one packed pair: with B1 = Mx^2 + My^2 + C1 and B2 = Vx + Vy + C2,
 //      SSIM = (1 - Md^2 / B1) (1 - Vd / B2),
@@ -33,12 +32,16 @@
 //  * Sums: the squared error (sci_sqerr.cuh) and 1 - SSIM are accumulated
 //    with compensated float32 additions over 8 rows and then added to float64.
 //
-// Measured at 2048 x 2048 x 8: 0.18 ms for the kernel (3.4 ms before), 58 %
-// of the issue slots; the packed float32 arithmetic of the windows bounds it
-// (about 100 instructions a pixel and lane, no spills at 3 blocks per SM; 4
-// blocks spill and take 0.20 ms).  Against float64, frames of 17 x 23 to
-// 2048 x 2048 with noise 0.003 to 0.1: mean SSIM at most 1.0e-8 off (2.4e-8
-// with float64 quotients of float32 moments), PSNR within 2e-14 dB.
+// Measured at 2048 x 2048 x 8: 0.205 ms for the kernel (3.4 ms in float64),
+// 0.18 of it without the squared error's third word and the windows' range
+// check; the packed float32 arithmetic of the windows bounds it (no spills at
+// 3 blocks per SM; 4 blocks spill).  Against float64 (rms over frames, this
+// kernel / float64 quotients of float32 moments): mean SSIM at noise 0.003 2e-12
+// to 2e-11 / 4e-10 to 2e-9, at 0.03 4e-11 to 3e-10 / 3e-10 to 2e-9 (64 x 64 to
+// 2048 x 2048).  The rounding of x + y is shared by the 49 windows of a pixel,
+// so between frames that differ more it averages out less than roundings of
+// each window's own: at 0.1 2e-10 to 1.4e-9 / 1e-11 to 1e-9, at 0.3 7e-11 to
+// 2e-9 / 1e-12 to 5e-10.  PSNR: as float64 gives it.
 #include <algorithm>
 
 #include "sci_sqerr.cuh"
@@ -230,7 +233,7 @@ __global__ void __launch_bounds__(WPB * 32, RESIDENT) k_frame_metrics(Metrics P)
             const float e1 = quotient(hi(S2), h1, P.c1, P.c1_lo);
             const float e2 = quotient(hi(V), h2, P.c2, P.c2_lo);
             const bool held = h1 + h2 < 1e30f;
-            ds.add(held ? fmaf(-e1, e2, e1 + e2) * win[k] : 0.f, 0.f);
+            ds.add(held ? fmaf(-e1, e2, e1 + e2) * win[k] : 0.f);
             if (!held && win[k] != 0.f) wide |= 1u << k;
         }
         return wide;

@@ -360,9 +360,9 @@ static void launch_admm_smem(const float *th, const float *bb, Mask<MODE> M, con
 // c = (y - yb)/phisum.  The x update x + lambda (c phi_b) is applied by the
 // TV kernel while it loads x (same arithmetic as k_proj_gap).
 // SQ: also adds sum (orig - x)^2 to *sq, the squared error of the iteration
-// that produced x.  In a pass of its own that read x once more and was a
-// launch: 15.8 us an iteration at 256 x 256 x 8 and 585 at 2048 x 2048 x 24
-// against 14.9 and 501 (12.2 and 416 without a ground truth).
+// that produced x: 16.0 us an iteration at 256 x 256 x 8 and 568 at 2048 x
+// 2048 x 24, 11.6 and 424 without a ground truth.  A pass of its own (k_sqerr)
+// reads x once more and is a launch: 4.5 and 165 us on top.
 template <int MODE, bool ACC, bool SQ>
 __global__ void __launch_bounds__(256) k_gap_resid_vec(
     const float *__restrict__ x, Mask<MODE> M, const float *__restrict__ y,
@@ -428,8 +428,8 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
 // yb = sum_b phi_b t_b and r_{k+1} = (y - yb) / (phisum + gamma).  With xo
 // it also writes x = t + lambda (r phi_b) of every frame (a second sweep).
 // SQ: also adds sum (orig - x)^2 to *sq, x stored or not (2048 x 2048 x 24: an
-// iteration 698 us with x stored for a pass of its own, 603 with it stored
-// here, 551 without).
+// iteration 586 us, 455 without a ground truth; a pass of its own takes 165
+// and x stored for it about 50).
 template <bool FIRST, bool WANT_X, bool SQ>
 __global__ void __launch_bounds__(256) k_admm_resid_vec(
     const float *__restrict__ tp, Mask<1> M, const float *__restrict__ y,
@@ -566,9 +566,9 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 // *out += sum (a - b)^2, the PSNR numerator of an iteration.  Few blocks: each
 // ends in one float64 atomic on the same word, and 2048 of them, with two
 // conversions and two float64 operations per element, were 12 us of a 256 x
-// 256 x 8 iteration (3.0 now: 8 bytes per element, launch and reduction).
-// At 2048 x 2048 x 24 the float64 pipe bounded it at 0.60 ms; now 0.13 ms,
-// 6.2 TB/s of the 805 MB it reads.
+// 256 x 8 iteration (4.5 now: launch and reduction).  At 2048 x 2048 x 24 the
+// float64 pipe bounded it at 0.74 ms; now issue does at 0.165 ms, 4.9 TB/s of
+// the 805 MB it reads.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_sqerr(const float *__restrict__ a,
                                                const float *__restrict__ b, int64_t n,

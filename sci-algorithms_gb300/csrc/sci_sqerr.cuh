@@ -1,9 +1,21 @@
-// Sum of squared float32 differences to float64 accuracy without float64
-// arithmetic in the loop (a GB300 SM does two float64 FMAs per clock against
-// 128 in float32): each square is an exact float32 product pair of an exact
-// difference pair, and the pairs are added with compensated float32
-// additions (relative error about 2^-45).  Differences whose squares float32
-// cannot hold so, and values that are not numbers, take a float64 branch.
+// Sum of squared float32 differences as accurate as float64 arithmetic gives
+// it, without float64 in the loop (a GB300 SM does two float64 FMAs per clock
+// against 128 in float32): the difference, its square and the additions are
+// carried with their rounding errors (error-free transformations: Knuth's
+// two-sum and two-difference, the product's error by FMA) in three float32
+// words.  Differences whose squares float32 cannot hold so, and values that
+// are not numbers, take a float64 branch.
+//
+// Two words are not enough, although a sum of random roundings would average
+// out: an odd square is 1 mod 8, so where its last bit is rounded off alone
+// the tie always falls to the even side below, and the sum lost 1 to 3e-15 of
+// itself at differences of 0.1 to 0.3.  Relative error of the sums of 32
+// elements that a thread adds before float64 takes over, differences of 0.03 /
+// 0.3 / a constant: 3e-17 / 5e-17 / 5e-17 (float64: 4e-17 / 1.1e-16 / 4.6e-16).
+//
+// What bounds it: issue, about 90 instructions for four elements (60 where
+// the vote below finds the differences exact).  k_sqerr at 2048 x 2048 x 8 and
+// x 24: 57 and 165 us (two words 47 and 136, float64 254 and 742).
 #pragma once
 
 #include "sci_common.cuh"
@@ -13,9 +25,9 @@ namespace sci {
 // Sum of terms with its rounding errors: hi + lo.
 struct Comp {
     float hi, lo;
-    __device__ __forceinline__ void add(float v, float v_lo) {
+    __device__ __forceinline__ void add(float v) {
         const float t = hi + v, z = t - hi;
-        lo += ((hi - (t - z)) + (v - z)) + v_lo;
+        lo += (hi - (t - z)) + (v - z);
         hi = t;
     }
     // An infinite total has no rounding error (inf - inf is not one).
@@ -26,11 +38,27 @@ struct Comp {
     }
 };
 
+// a + b rounded; err the rest, exactly.
+__device__ __forceinline__ f2 two_sum(f2 a, f2 b, f2 &err) {
+    const f2 t = add2(a, b), z = sub2(t, a);
+    err = add2(sub2(a, sub2(t, z)), sub2(b, z));
+    return t;
+}
+
+// a b rounded; err the rest, exactly.  The product is formed by halves: ptxas
+// contracts a packed product and a packed sum into an FMA, explicit rounding or
+// not, and the rest needs the rounded product.
+__device__ __forceinline__ f2 two_mul(f2 a, f2 b, f2 &err) {
+    const f2 t = mk2(__fmul_rn(lo(a), lo(b)), __fmul_rn(hi(a), hi(b)));
+    err = fma2(a, b, sub2(mk2(0.f, 0.f), t));
+    return t;
+}
+
 struct SquareSum {
-    Comp c;
+    f2 s0, s1, s2;  // sum of the even and the odd elements, in three words
     double wide;
     __device__ __forceinline__ void clear() {
-        c = {0.f, 0.f};
+        s0.v = s1.v = s2.v = 0ull;
         wide = 0.0;
     }
     // Adds (x_k - y_k)^2, given d_k = x_k - y_k rounded, k < 4.  Called by
@@ -56,25 +84,38 @@ struct SquareSum {
             }
             return;
         }
-        // x - y = d + dl exactly; d^2 = t + its rounding error.  The
-        // products are scalar: ptxas contracts a packed product and a packed
-        // sum into an FMA, explicit rounding or not, and the error terms
-        // need the rounded product.
-        f2 t[2], e[2];
+        // x - y = d + dl exactly, (d + dl)^2 = d^2 + 2 d dl + dl^2: words t (of
+        // d^2), m (about 2^-24 of it) and l (2^-48)
+        f2 D[2], dl[2], t[2], m[2], l[2];
+        unsigned rest = 0u;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const float d0 = d[2 * h], d1 = d[2 * h + 1];
             const f2 X = mk2(x[2 * h], x[2 * h + 1]), Y = mk2(y[2 * h], y[2 * h + 1]);
-            const f2 D = mk2(d0, d1), z = sub2(D, X);
-            const f2 dl = sub2(sub2(X, sub2(D, z)), add2(Y, z));
-            t[h] = mk2(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-            e[h] = fma2(add2(D, D), dl, fma2(D, D, sub2(mk2(0.f, 0.f), t[h])));
+            D[h] = mk2(d[2 * h], d[2 * h + 1]);
+            const f2 z = sub2(D[h], X);
+            dl[h] = sub2(sub2(X, sub2(D[h], z)), add2(Y, z));
+            t[h] = two_mul(D[h], D[h], m[h]);
+            l[h].v = 0ull;
+            rest |= __float_as_uint(lo(dl[h])) | __float_as_uint(hi(dl[h]));
         }
-        // t[0] + t[1], exactly as a sum and its error, then into the total
-        const f2 u = add2(t[0], t[1]), z = sub2(u, t[0]);
-        const f2 ue = add2(add2(sub2(t[0], sub2(u, z)), sub2(t[1], z)), add2(e[0], e[1]));
-        c.add(lo(u), lo(ue));
-        c.add(hi(u), hi(ue));
+        // values within a factor of two of each other differ exactly: a vote
+        // mostly leaves this out where the frames agree
+        if (__any_sync(__activemask(), (rest << 1) != 0u)) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                f2 pe, me;
+                const f2 p = two_mul(add2(D[h], D[h]), dl[h], pe);
+                m[h] = two_sum(m[h], p, me);
+                l[h] = add2(fma2(dl[h], dl[h], pe), me);
+            }
+        }
+        // the two pairs to one, then into the total
+        f2 e0, e1, e2, e3, e4;
+        const f2 tt = two_sum(t[0], t[1], e0);
+        const f2 mm = two_sum(e0, two_sum(m[0], m[1], e1), e2);
+        s0 = two_sum(s0, tt, e0);
+        s1 = two_sum(s1, two_sum(e0, mm, e3), e4);
+        s2 = add2(s2, add2(add2(add2(e1, e2), add2(e3, e4)), add2(l[0], l[1])));
     }
     __device__ __forceinline__ void add4(float4 a, float4 b) {
         const float x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
@@ -82,8 +123,10 @@ struct SquareSum {
         add4(x, y, d);
     }
     __device__ __forceinline__ double take() {
-        const double r = c.take() + wide;
-        wide = 0.0;
+        const double r = (((double)lo(s0) + (double)hi(s0)) +
+                          (((double)lo(s1) + (double)hi(s1)) + (double)(lo(s2) + hi(s2)))) +
+                         wide;
+        clear();
         return r;
     }
 };

@@ -1,5 +1,6 @@
 """GPU parity of the mask operators and projections against the oracle."""
 import ctypes
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -253,3 +254,28 @@ def test_sqerr_accum_is_exact_to_float64(n, offset):
              torch.cuda.current_stream().cuda_stream)
         ref = 2.0 * scale * scale + ((x.double() - y.double()) ** 2).sum().item()
         assert abs(out.item() / ref - 1) < 1e-12
+
+
+# No bias: 2048 elements (one block) at a time, of pairs whose difference
+# float32 rounds.  Its square is the square of the rounded difference, twice
+# the product with the rounding error and that error's square, the last 2^-50
+# of the whole and always of one sign.  Roundings of either sign are at most
+# 2^-49 of an element and 2^-53 of a sum and average out over 512 sums of 2048
+# elements (2^-59), so the mean relative error is below 2^-53 (1.1e-16).
+@pytest.mark.parametrize("low,high", [(0.25, 0.5), (0.5, 1.0), (0.3, 0.9)])
+def test_sqerr_accum_has_no_bias(low, high):
+    from sci_algorithms_gb300._lib import call
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = 2.0 ** -7 * torch.rand((512, 2048), device="cuda", generator=g)
+    b = low + (high - low) * torch.rand((512, 2048), device="cuda", generator=g)
+    out = torch.zeros(512, dtype=torch.float64, device="cuda")
+    for i in range(512):
+        call("sci_sqerr_accum", a[i].data_ptr(), b[i].data_ptr(), 2048, out[i:].data_ptr(),
+             torch.cuda.current_stream().cuda_stream)
+    # the differences are multiples of 2^-40, exact in float64: integer squares
+    d = (a.double() - b.double()).cpu().numpy() * 2.0 ** 40
+    err = []
+    for i in range(512):
+        exact = Fraction(sum(int(v) ** 2 for v in d[i]), 2 ** 80)
+        err.append(float(Fraction(out[i].item()) / exact - 1))
+    assert abs(np.mean(err)) < 2.0 ** -53, np.mean(err)

@@ -44,17 +44,17 @@ __device__ __forceinline__ void resid_task(const Item &I, const tv::Pass &P, int
     const int64_t p = (int64_t)tile * QP_T + lane * 4;
     if (p >= hw) return;  // hw % 4 == 0: all 4 pixels are inside
     const int B = I.B;
-    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(I.bits + p));
+    const uint4 w = *reinterpret_cast<const uint4 *>(I.bits + p);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int b = 0; b < B; ++b) {
-        const float4 v = ldg4(P.f + b * hw + p);
+        const float4 v = ld4(P.f + b * hw + p);
         s.x = fmaf(v.x, bitf(w.x, b), s.x);
         s.y = fmaf(v.y, bitf(w.y, b), s.y);
         s.z = fmaf(v.z, bitf(w.z, b), s.z);
         s.w = fmaf(v.w, bitf(w.w, b), s.w);
     }
-    const float4 yv = ldg4(I.y + p), ps = ldg4(I.phisum + p);
+    const float4 yv = ld4(I.y + p), ps = ld4(I.phisum + p);
     float4 r;
     if (ACC) {
         float4 tt = *reinterpret_cast<const float4 *>(I.y1 + p);
@@ -116,7 +116,7 @@ __device__ __forceinline__ void tv_task(const tv::Pass &P, int frame, int chunk,
 __device__ __forceinline__ int warp_find(const int *prefix, int n, int g, int lane) {
     int i = 0;
     for (int q = 0; q < n; q += 32)
-        i += __popc(__ballot_sync(0xffffffffu, q + lane < n && __ldg(prefix + q + lane + 1) <= g));
+        i += __popc(__ballot_sync(0xffffffffu, q + lane < n && prefix[q + lane + 1] <= g));
     return i;
 }
 

@@ -95,9 +95,8 @@ __global__ void k_cassi_phisum(const float *__restrict__ phi, float *__restrict_
 // 28 against 5.5.
 template <bool ACC>
 __global__ void __launch_bounds__(128) k_cassi_resid(
-    const float *__restrict__ x, const float *__restrict__ phi, const float *__restrict__ y,
-    float *__restrict__ y1, const float *__restrict__ ps, float *__restrict__ r, int L, int H,
-    int W, int step, double *__restrict__ zero, int nzero) {
+    const float *x, const float *phi, const float *y, float *__restrict__ y1, const float *ps,
+    float *__restrict__ r, int L, int H, int W, int step, double *__restrict__ zero, int nzero) {
     constexpr int G = 8;
     grid_dep_wait();
     if (blockIdx.x == 0 && blockIdx.y == 0)  // the next TV pass's stop-test sums
@@ -118,8 +117,8 @@ __global__ void __launch_bounds__(128) k_cassi_resid(
 #pragma unroll
             for (int u = 0; u < G; ++u)
                 if (b + u <= b1) {
-                    xv[u] = __ldg(xp + (b + u) * (hw - step));
-                    m[u] = __ldg(mp - (b + u) * step);
+                    xv[u] = xp[(b + u) * (hw - step)];
+                    m[u] = mp[-(b + u) * step];
                 }
 #pragma unroll
             for (int u = 0; u < G; ++u)
@@ -158,9 +157,9 @@ __global__ void k_cassi_update(const float *__restrict__ x, const float *__restr
 // leaves the chip.  Needs Wd floats of shared memory.
 template <bool ACC>
 __global__ void __launch_bounds__(1024) k_cassi_proj_rows(
-    const float *__restrict__ x, const float *__restrict__ phi, const float *__restrict__ y,
-    float *__restrict__ y1, const float *__restrict__ ps, float *__restrict__ xo, float lam,
-    int L, int H, int W, int step, double *__restrict__ zero, int nzero) {
+    const float *x, const float *phi, const float *y, float *__restrict__ y1, const float *ps,
+    float *__restrict__ xo, float lam, int L, int H, int W, int step, double *__restrict__ zero,
+    int nzero) {
     extern __shared__ float rs[];
     grid_dep_wait();
     if (blockIdx.x == 0)  // the next TV pass's stop-test sums
@@ -175,7 +174,7 @@ __global__ void __launch_bounds__(1024) k_cassi_proj_rows(
             float s = 0.f;
             for (int b = b0; b <= b1; ++b) {
                 const int64_t p = (int64_t)h * W + (wd - step * b);
-                s = fmaf(__ldg(x + b * hw + p), __ldg(phi + p), s);
+                s = fmaf(x[b * hw + p], phi[p], s);
             }
             if (ACC) {
                 const float t = y1[i] + (y[i] - s);
@@ -189,7 +188,7 @@ __global__ void __launch_bounds__(1024) k_cassi_proj_rows(
         for (int e = threadIdx.x; e < L * W; e += blockDim.x) {
             const int b = e / W, w = e - b * W;
             const int64_t p = (int64_t)h * W + w;
-            xo[b * hw + p] = fmaf(lam, rs[w + step * b] * __ldg(phi + p), __ldg(x + b * hw + p));
+            xo[b * hw + p] = fmaf(lam, rs[w + step * b] * phi[p], x[b * hw + p]);
         }
         __syncthreads();
     }

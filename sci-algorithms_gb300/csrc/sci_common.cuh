@@ -46,6 +46,12 @@ constexpr int kSMs = 152;  // GB300: 2 dies x 76 SMs
 // returns once the predecessor grid has completed and its writes are
 // visible (a no-op for a normal launch).  This hides the launch gap between
 // consecutive kernels.  SCI_PDL=0 launches them normally.
+//
+// Such a kernel may have begun while its input is still written, so that
+// input is not read-only for its lifetime: these kernels read the arrays that
+// an earlier kernel may write with plain loads (ld4 and C++ accesses) through
+// pointers without __restrict__, never with __ldg, whose cache need not see
+// those writes and whose result the compiler may take as invariant.
 bool pdl_enabled();
 
 template <typename... K, typename... A>
@@ -78,6 +84,10 @@ __device__ __forceinline__ void grid_dep_launch() {
 // ------------------------------------------------------------- device side
 __device__ __forceinline__ float4 ldg4(const float *p) {
     return __ldg(reinterpret_cast<const float4 *>(p));
+}
+// a plain load (of memory that a kernel still running may have written)
+__device__ __forceinline__ float4 ld4(const float *p) {
+    return *reinterpret_cast<const float4 *>(p);
 }
 __device__ __forceinline__ void st4(float *p, float4 v) {
     *reinterpret_cast<float4 *>(p) = v;

@@ -68,6 +68,7 @@ static inline dim3 grid_for(int64_t n, int threads) {
 
 // --------------------------------------------------------- mask helpers
 // MODE 0: float mask phi[b][p];  MODE 1: packed bits word[p], bit b.
+// Plain loads: kernels that wait for their predecessor use them too.
 template <int MODE>
 struct Mask;
 template <>
@@ -75,10 +76,10 @@ struct Mask<0> {
     const float *phi;
     int64_t hw;
     __device__ __forceinline__ float4 at4(int b, int64_t p, uint4) const {
-        return ldg4(phi + (int64_t)b * hw + p);
+        return ld4(phi + (int64_t)b * hw + p);
     }
     __device__ __forceinline__ float at1(int b, int64_t p, uint32_t) const {
-        return __ldg(phi + (int64_t)b * hw + p);
+        return phi[(int64_t)b * hw + p];
     }
     __device__ __forceinline__ uint4 word4(int64_t) const { return make_uint4(0, 0, 0, 0); }
     __device__ __forceinline__ uint32_t word1(int64_t) const { return 0u; }
@@ -95,9 +96,9 @@ struct Mask<1> {
     }
     __device__ __forceinline__ float at1(int b, int64_t, uint32_t w) const { return bit(w, b); }
     __device__ __forceinline__ uint4 word4(int64_t p) const {
-        return __ldg(reinterpret_cast<const uint4 *>(bits + p));
+        return *reinterpret_cast<const uint4 *>(bits + p);
     }
-    __device__ __forceinline__ uint32_t word1(int64_t p) const { return __ldg(bits + p); }
+    __device__ __forceinline__ uint32_t word1(int64_t p) const { return bits[p]; }
 };
 
 // ------------------------------------------------------------------- A_
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(256) k_proj_gap_vec(
         const float4 yv = ldg4(y + p), ps = ldg4(phisum + p);
         float4 r;
         if (ACC) {
-            float4 t = ldg4(y1 + p);
+            float4 t = ld4(y1 + p);
             t.x = t.x + (yv.x - s.x);
             t.y = t.y + (yv.y - s.y);
             t.z = t.z + (yv.z - s.z);
@@ -365,10 +366,9 @@ static void launch_admm_smem(const float *th, const float *bb, Mask<MODE> M, con
 // reads x once more and is a launch: 4.5 and 165 us on top.
 template <int MODE, bool ACC, bool SQ>
 __global__ void __launch_bounds__(256) k_gap_resid_vec(
-    const float *__restrict__ x, Mask<MODE> M, const float *__restrict__ y,
-    float *__restrict__ y1, const float *__restrict__ phisum, float *__restrict__ c, int B,
-    int64_t hw, double *__restrict__ rn, double *__restrict__ zero, int nzero, int rev,
-    const float *__restrict__ orig, double *__restrict__ sq) {
+    const float *x, Mask<MODE> M, const float *y, float *__restrict__ y1, const float *phisum,
+    float *__restrict__ c, int B, int64_t hw, double *__restrict__ rn, double *__restrict__ zero,
+    int nzero, int rev, const float *orig, double *__restrict__ sq) {
     grid_dep_wait();
     if (gridDim.x > kSMs * 8) grid_dep_launch();
     if (blockIdx.x == 0)  // the next TV pass's stop-test sums
@@ -384,19 +384,19 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
         for (int b = 0; b < B; ++b) {
-            const float4 a = ldg4(x + b * hw + p), m = M.at4(b, p, w);
+            const float4 a = ld4(x + b * hw + p), m = M.at4(b, p, w);
             s.x = fmaf(a.x, m.x, s.x);
             s.y = fmaf(a.y, m.y, s.y);
             s.z = fmaf(a.z, m.z, s.z);
             s.w = fmaf(a.w, m.w, s.w);
-            if (SQ) se.add4(ldg4(orig + b * hw + p), a);
+            if (SQ) se.add4(ld4(orig + b * hw + p), a);
             if (SQ && (b & 7) == 7) sacc += se.take();
         }
         if (SQ) sacc += se.take();
-        const float4 yv = ldg4(y + p), ps = ldg4(phisum + p);
+        const float4 yv = ld4(y + p), ps = ld4(phisum + p);
         float4 r;
         if (ACC) {
-            float4 t = ldg4(y1 + p);
+            float4 t = ld4(y1 + p);
             t.x = t.x + (yv.x - s.x);
             t.y = t.y + (yv.y - s.y);
             t.z = t.z + (yv.z - s.z);
@@ -432,16 +432,15 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
 // and x stored for it about 50).
 template <bool FIRST, bool WANT_X, bool SQ>
 __global__ void __launch_bounds__(256) k_admm_resid_vec(
-    const float *__restrict__ tp, Mask<1> M, const float *__restrict__ y,
-    const float *__restrict__ phisum, float *__restrict__ rnew, float *__restrict__ xo, float lam,
-    float gamma, int B, int64_t hw, double *__restrict__ rn, double *__restrict__ zero,
-    int nzero, int rev, const float *__restrict__ orig, double *__restrict__ sq) {
+    const float *tp, Mask<1> M, const float *y, const float *phisum, float *__restrict__ rnew,
+    float *__restrict__ xo, float lam, float gamma, int B, int64_t hw, double *__restrict__ rn,
+    double *__restrict__ zero, int nzero, int rev, const float *orig, double *__restrict__ sq) {
     grid_dep_wait();
     if (gridDim.x > kSMs * 8) grid_dep_launch();
     if (blockIdx.x == 0)  // the next TV pass's stop-test sums
         for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0.0;
     auto tload = [&](int64_t o) {
-        const float4 a = ldg4(tp + o);
+        const float4 a = ld4(tp + o);
         return FIRST ? make_float4(a.x + 0.f, a.y + 0.f, a.z + 0.f, a.w + 0.f) : a;
     };
     const int64_t n4 = hw >> 2;
@@ -462,7 +461,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
             s.z = fmaf(t.z, m.z, s.z);
             s.w = fmaf(t.w, m.w, s.w);
         }
-        const float4 yv = ldg4(y + p), ps = ldg4(phisum + p);
+        const float4 yv = ld4(y + p), ps = ld4(phisum + p);
         const float4 r = make_float4(__fdiv_rn(yv.x - s.x, ps.x + gamma),
                                      __fdiv_rn(yv.y - s.y, ps.y + gamma),
                                      __fdiv_rn(yv.z - s.z, ps.z + gamma),
@@ -478,7 +477,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
                     make_float4(fmaf(lam, r.x * m.x, t.x), fmaf(lam, r.y * m.y, t.y),
                                 fmaf(lam, r.z * m.z, t.z), fmaf(lam, r.w * m.w, t.w));
                 if (WANT_X) st4(xo + b * hw + p, xv);
-                if (SQ) se.add4(ldg4(orig + b * hw + p), xv);
+                if (SQ) se.add4(ld4(orig + b * hw + p), xv);
                 if (SQ && (b & 7) == 7) sacc += se.take();
             }
             if (SQ) sacc += se.take();
@@ -570,8 +569,7 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 // float64 pipe bounded it at 0.74 ms; now issue does at 0.165 ms, 4.9 TB/s of
 // the 805 MB it reads.
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_sqerr(const float *__restrict__ a,
-                                               const float *__restrict__ b, int64_t n,
+__global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, int64_t n,
                                                double *out) {
     grid_dep_wait();
     SquareSum s;
@@ -582,14 +580,14 @@ __global__ void __launch_bounds__(256) k_sqerr(const float *__restrict__ a,
          i += 4 * (int64_t)gridDim.x * blockDim.x) {
         float x[4], y[4], d[4];
         if (VEC) {
-            const float4 u = ldg4(a + i), v = ldg4(b + i);
+            const float4 u = ld4(a + i), v = ld4(b + i);
             x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
             y[0] = v.x, y[1] = v.y, y[2] = v.z, y[3] = v.w;
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                x[k] = i + k < n ? __ldg(a + i + k) : 0.f;
-                y[k] = i + k < n ? __ldg(b + i + k) : 0.f;
+                x[k] = i + k < n ? a[i + k] : 0.f;
+                y[k] = i + k < n ? b[i + k] : 0.f;
             }
         }
 #pragma unroll

@@ -134,3 +134,46 @@ def test_cassi_projection_on_load_is_bitwise_equal(monkeypatch, H, W, L, step, a
             out.append(s.run(y).clone())
     for x in out[1:]:
         assert torch.equal(out[0], x)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_cassi_bad_detector_pixel_on_the_fused_path(monkeypatch, bad):
+    """A detector pixel that is not finite spreads as through the projection
+    kernel."""
+    H, W, L, step = 50, 70, 4, 2
+    rng = np.random.default_rng(4)
+    phi = torch.from_numpy((rng.random((H, W)) < 0.5).astype(np.float32)).cuda()
+    op = sci.CassiOperator(phi, L, step)
+    y = torch.from_numpy(rng.random((H, op.Wd)).astype(np.float32)).cuda()
+    y[20, 30] = bad
+    y[H - 1, op.Wd - 1] = bad
+    out = []
+    for fused in ("0", "1"):
+        monkeypatch.setenv("SCI_FUSED_PROJ", fused)
+        out.append(sci.CassiSolver(op, 2, 0.8, 0.1, 5, eps=0.0).run(y).clone())
+    assert torch.equal(torch.isnan(out[0]), torch.isnan(out[1]))
+    assert torch.equal(torch.nan_to_num(out[0]), torch.nan_to_num(out[1]))
+
+
+# Cubes whose windows are too many for the small window shape: the projection
+# on load in windows of 64 x 48.
+@pytest.mark.parametrize("H,W,L,step", [(130, 177, 28, 2), (49, 66, 80, 1), (45, 61, 152, 3)])
+def test_cassi_projection_on_load_in_large_windows(monkeypatch, H, W, L, step):
+    test_cassi_projection_on_load_is_bitwise_equal(monkeypatch, H, W, L, step, True, 0.05, 5)
+
+
+# The row-fused projection, 512 and 1024 threads per row, where the projection
+# is not applied on load (SCI_FUSED_PROJ=0; large cubes take this route).
+@pytest.mark.parametrize("accelerate", [True, False])
+@pytest.mark.parametrize("threads", ["128", "512", "1024"])
+def test_cassi_row_projection_kernel(monkeypatch, accelerate, threads):
+    cube, phi, y = cassi_problem()
+    op = sci.CassiOperator(phi, 28, 2)
+    yd = torch.from_numpy(y).float().to(op.dev)
+    monkeypatch.setenv("SCI_FUSED_PROJ", "0")
+    monkeypatch.setenv("SCI_CASSI_ROWT", threads)
+    out = []
+    for rows in ("0", "1"):
+        monkeypatch.setenv("SCI_CASSI_ROWS", rows)
+        out.append(sci.CassiSolver(op, 12, 1.0, 0.05, 5, accelerate=accelerate).run(yd).clone())
+    assert torch.equal(*out)

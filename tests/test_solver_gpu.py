@@ -466,3 +466,43 @@ def test_bad_measurement_pixel_on_the_fused_path(monkeypatch, gray, tvm, bad, W)
     assert not torch.isfinite(out[0]).all()
     for i in range(2, 6):
         assert same(out[i % 2], out[i])
+
+
+def test_squared_error_of_bad_values():
+    """The residual passes' squared error and the kernel of its own, where an
+    element is not finite or its square is beyond float32."""
+    from sci_algorithms_gb300._lib import call
+    a = torch.rand(4096, device="cuda")
+    for bad, want in ((float("nan"), np.isnan), (float("inf"), np.isposinf),
+                      (3e38, lambda v: np.isclose(v, 9e76, rtol=1e-6)),
+                      (1e-38, np.isfinite)):
+        for at in (0, 1234, 4095):
+            b = a.clone()
+            b[at] = bad
+            out = torch.zeros(1, dtype=torch.float64, device="cuda")
+            call("sci_sqerr_accum", a.data_ptr(), b.data_ptr(), 4096, out.data_ptr(),
+                 _dev.stream_handle())
+            assert want(out.item()), (bad, at, out.item())
+
+
+# The projections on load in windows of 64 x 48 (more than 300 of them; fewer
+# run in windows of 64 x 32): float masks, packed masks and ADMM's t output.
+@pytest.mark.parametrize("H,W,B,kind,gray", [(130, 180, 32, "gap", False), (49, 68, 80, "gap", True),
+                                             (130, 180, 24, "gap", True),
+                                             (130, 180, 32, "admm", False)])
+@pytest.mark.parametrize("K", [2, 5])
+@pytest.mark.parametrize("eps", [0.0, 0.02])
+def test_projection_on_load_in_large_windows(monkeypatch, H, W, B, kind, gray, K, eps):
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    mask = torch.rand(H, W, B, device="cuda", generator=g)
+    if not gray:
+        mask = (mask < 0.5).float()
+    op = sci.MaskOperator(mask)
+    y = op.phi.sum(0) * torch.rand(H, W, device="cuda", generator=g)
+    out = []
+    for tile in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        s = sci.Solver(op, kind, 5, 0.9, 0.1, K, eps=eps)
+        out.append((s.run(y, tv_steps=True).clone(), s.tv_steps.clone()))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1], out[1][1])

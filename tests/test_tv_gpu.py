@@ -239,3 +239,73 @@ def test_tv_tile_unaligned_and_resid(H, W, monkeypatch):
                 assert torch.equal(r, u - f)
                 ref = ref or {}
                 assert torch.equal(ref.setdefault(K, u), u)
+
+
+# The shape a call takes by itself, against the row pipelines and the oracle.
+@pytest.mark.parametrize("H,W,F,K", [(517, 643, 4, 9), (300, 500, 6, 5), (64, 96, 8, 30)])
+def test_tv_default_route(H, W, F, K, monkeypatch):
+    f = smooth_frames(H, W, F, seed=H + K)
+    fp = _dev.planar(f)
+    ref, steps_ref, _ = tv_chambolle_frames(f, 0.1, n_iter_max=K)
+    u, steps, _ = _tv_env(monkeypatch, fp, 0.1, K, 2e-4, "1")
+    assert np.max(np.abs(_dev.unplanar(u, f) - ref)) < ATOL
+    assert list(steps) == steps_ref
+    monkeypatch.setenv("SCI_TV_TILE", "0")
+    u0, s0, _ = _tv_env(monkeypatch, fp, 0.1, K, 2e-4, "1")
+    assert torch.equal(u, u0)
+    assert list(steps) == list(s0)
+
+
+# More than 300 windows of 64 x 48 (56 x 40 owned; 2 x 8 pixels per thread):
+# fewer run in windows of 64 x 32, which the shapes above all do.  Many small
+# frames reach every edge of the large ones: frames of one window, of its
+# size, one more, its halo; odd widths; one to eight passes.
+@pytest.mark.parametrize("H,W,F", [(5, 7, 301), (47, 63, 301), (48, 64, 302), (49, 64, 151),
+                                   (48, 65, 152), (49, 66, 80), (44, 121, 110), (88, 120, 76),
+                                   (89, 119, 51), (90, 181, 40), (130, 177, 20)])
+@pytest.mark.parametrize("K", [2, 4, 5, 6, 9, 14])
+def test_tv_large_windows_bitwise_equal_pipeline(H, W, F, K, monkeypatch):
+    test_tv_tile_bitwise_equals_pipeline(H, W, F, K, monkeypatch)
+
+
+@pytest.mark.parametrize("H,W,F", [(50, 66, 90), (97, 131, 51)])
+def test_tv_large_windows_unaligned_and_resid(H, W, F, monkeypatch):
+    f = _dev.planar(smooth_frames(H, W, F, seed=5))
+    store = torch.zeros(f.numel() + 1, device="cuda")
+    g = store[1:].view(f.shape)  # 4-byte aligned rows
+    g.copy_(f)
+    ref = {}
+    for tile in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        for src in (f, g):
+            for K in (5, 11):
+                r = torch.full_like(f, 7.0)
+                u = sci.tv_frames(src, 0.2, K, resid=r)
+                assert torch.equal(r, u - f)
+                assert torch.equal(ref.setdefault(K, u), u)
+
+
+# The lean row pipeline itself (SCI_TV_TILE=0: frames of this size run on
+# tiles otherwise).
+@pytest.mark.parametrize("H,W,F", [(64, 1024, 3), (257, 516, 2), (33, 640, 5)])
+def test_tv_lean_pipeline_matches_oracle(H, W, F, monkeypatch):
+    monkeypatch.setenv("SCI_TV_TILE", "0")
+    test_tv_slim_matches_oracle(H, W, F, monkeypatch)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3e38])
+@pytest.mark.parametrize("H,W,F", [(50, 67, 2), (50, 66, 90), (130, 180, 2)])
+@pytest.mark.parametrize("K", [2, 5, 9])
+def test_tv_tile_bad_pixels_spread_as_in_the_pipeline(H, W, F, K, bad, monkeypatch):
+    f = _dev.planar(smooth_frames(H, W, F, seed=1)).clone()
+    f[0, H // 2, W // 2] = bad
+    f[0, H - 1, W - 1] = bad
+    f[1, 0, 0] = bad
+    f[1, H - 1, 3] = bad
+    out = []
+    for tile in ("0", "1"):
+        monkeypatch.setenv("SCI_TV_TILE", tile)
+        out.append(sci.tv_frames(f, 0.1, K, 0.0))
+    a, b = out
+    assert torch.equal(torch.isnan(a), torch.isnan(b))
+    assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))

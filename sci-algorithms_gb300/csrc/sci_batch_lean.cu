@@ -44,7 +44,7 @@ __device__ __forceinline__ void resid_task(const Item &I, const tv::Pass &P, int
     const int64_t p = (int64_t)tile * QP_T + lane * 4;
     if (p >= hw) return;  // hw % 4 == 0: all 4 pixels are inside
     const int B = I.B;
-    const uint4 w = *reinterpret_cast<const uint4 *>(I.bits + p);
+    const uint4 w = ld4(I.bits + p);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int b = 0; b < B; ++b) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ int warp_find(const int *prefix, int n, int g, int la
 
 // One phase of iteration k over all items as a launch of its own.
 template <bool ACC>
-__global__ void __launch_bounds__(tv::WPB * 32) k_batch_resid(const Table *__restrict__ T, int k) {
+__global__ void __launch_bounds__(tv::WPB * 32, 4) k_batch_resid(const Table *__restrict__ T, int k) {
     grid_dep_wait();
     if (gridDim.x > kSMs * 8) grid_dep_launch();
     const int lane = threadIdx.x & 31, g = blockIdx.x * tv::WPB + (threadIdx.x >> 5);

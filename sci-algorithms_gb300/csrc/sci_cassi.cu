@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(128) k_cassi_resid(
     band_range(wd, W, L, step, b0, b1);
     for (int h = blockIdx.y; h < H; h += gridDim.y) {
         const int64_t i = (int64_t)h * Wd + wd;
-        const float yv = y[i], pv = ps[i], tv = ACC ? y1[i] : 0.f;
+        const float yv = ld1(y + i), pv = ld1(ps + i), tv = ACC ? ld1(y1 + i) : 0.f;
         const float *xp = x + (int64_t)h * W + wd, *mp = phi + (int64_t)h * W + wd;
         float s = 0.f;
         for (int b = b0; b <= b1; b += G) {
@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(128) k_cassi_resid(
 #pragma unroll
             for (int u = 0; u < G; ++u)
                 if (b + u <= b1) {
-                    xv[u] = xp[(b + u) * (hw - step)];
-                    m[u] = mp[-(b + u) * step];
+                    xv[u] = ld1(xp + (b + u) * (hw - step));
+                    m[u] = ld1(mp - (b + u) * step);
                 }
 #pragma unroll
             for (int u = 0; u < G; ++u)
@@ -174,21 +174,22 @@ __global__ void __launch_bounds__(1024) k_cassi_proj_rows(
             float s = 0.f;
             for (int b = b0; b <= b1; ++b) {
                 const int64_t p = (int64_t)h * W + (wd - step * b);
-                s = fmaf(x[b * hw + p], phi[p], s);
+                s = fmaf(ld1(x + b * hw + p), ld1(phi + p), s);
             }
             if (ACC) {
-                const float t = y1[i] + (y[i] - s);
+                const float t = ld1(y1 + i) + (ld1(y + i) - s);
                 y1[i] = t;
-                rs[wd] = __fdiv_rn(t - s, ps[i]);
+                rs[wd] = __fdiv_rn(t - s, ld1(ps + i));
             } else {
-                rs[wd] = __fdiv_rn(y[i] - s, ps[i]);
+                rs[wd] = __fdiv_rn(ld1(y + i) - s, ld1(ps + i));
             }
         }
         __syncthreads();
         for (int e = threadIdx.x; e < L * W; e += blockDim.x) {
             const int b = e / W, w = e - b * W;
             const int64_t p = (int64_t)h * W + w;
-            xo[b * hw + p] = fmaf(lam, rs[w + step * b] * phi[p], x[b * hw + p]);
+            xo[b * hw + p] =
+                fmaf(lam, rs[w + step * b] * ld1(phi + p), ld1(x + b * hw + p));
         }
         __syncthreads();
     }

@@ -49,8 +49,8 @@ constexpr int kSMs = 152;  // GB300: 2 dies x 76 SMs
 //
 // Such a kernel may have begun while its input is still written, so that
 // input is not read-only for its lifetime: these kernels read the arrays that
-// an earlier kernel may write with plain loads (ld4 and C++ accesses) through
-// pointers without __restrict__, never with __ldg, whose cache need not see
+// an earlier kernel may write with plain loads (ld1, ld4, C++ accesses through
+// pointers without __restrict__), never with __ldg, whose cache need not see
 // those writes and whose result the compiler may take as invariant.
 bool pdl_enabled();
 
@@ -85,9 +85,27 @@ __device__ __forceinline__ void grid_dep_launch() {
 __device__ __forceinline__ float4 ldg4(const float *p) {
     return __ldg(reinterpret_cast<const float4 *>(p));
 }
-// a plain load (of memory that a kernel still running may have written)
+// Plain loads, in program order, for kernels that wait for their predecessor.
+// (As C++ accesses through pointers that may alias what the kernel stores, the
+// compiler had fewer of them in flight: up to 10 % of an iteration.)
+__device__ __forceinline__ float ld1(const float *p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float4 ld4(const float *p) {
-    return *reinterpret_cast<const float4 *>(p);
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld4(const uint32_t *p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
 }
 __device__ __forceinline__ void st4(float *p, float4 v) {
     *reinterpret_cast<float4 *>(p) = v;

@@ -68,7 +68,8 @@ static inline dim3 grid_for(int64_t n, int threads) {
 
 // --------------------------------------------------------- mask helpers
 // MODE 0: float mask phi[b][p];  MODE 1: packed bits word[p], bit b.
-// Plain loads: kernels that wait for their predecessor use them too.
+// Mask: plain loads, for the kernels that wait for their predecessor;
+// ConstMask: read-only loads, for the others.
 template <int MODE>
 struct Mask;
 template <>
@@ -78,11 +79,7 @@ struct Mask<0> {
     __device__ __forceinline__ float4 at4(int b, int64_t p, uint4) const {
         return ld4(phi + (int64_t)b * hw + p);
     }
-    __device__ __forceinline__ float at1(int b, int64_t p, uint32_t) const {
-        return phi[(int64_t)b * hw + p];
-    }
     __device__ __forceinline__ uint4 word4(int64_t) const { return make_uint4(0, 0, 0, 0); }
-    __device__ __forceinline__ uint32_t word1(int64_t) const { return 0u; }
 };
 template <>
 struct Mask<1> {
@@ -94,11 +91,28 @@ struct Mask<1> {
     __device__ __forceinline__ float4 at4(int b, int64_t, uint4 w) const {
         return make_float4(bit(w.x, b), bit(w.y, b), bit(w.z, b), bit(w.w, b));
     }
+    __device__ __forceinline__ uint4 word4(int64_t p) const { return ld4(bits + p); }
+};
+
+template <int MODE>
+struct ConstMask;
+template <>
+struct ConstMask<0> : Mask<0> {
+    __device__ __forceinline__ float4 at4(int b, int64_t p, uint4) const {
+        return ldg4(phi + (int64_t)b * hw + p);
+    }
+    __device__ __forceinline__ float at1(int b, int64_t p, uint32_t) const {
+        return __ldg(phi + (int64_t)b * hw + p);
+    }
+    __device__ __forceinline__ uint32_t word1(int64_t) const { return 0u; }
+};
+template <>
+struct ConstMask<1> : Mask<1> {
     __device__ __forceinline__ float at1(int b, int64_t, uint32_t w) const { return bit(w, b); }
     __device__ __forceinline__ uint4 word4(int64_t p) const {
-        return *reinterpret_cast<const uint4 *>(bits + p);
+        return __ldg(reinterpret_cast<const uint4 *>(bits + p));
     }
-    __device__ __forceinline__ uint32_t word1(int64_t p) const { return bits[p]; }
+    __device__ __forceinline__ uint32_t word1(int64_t p) const { return __ldg(bits + p); }
 };
 
 // ------------------------------------------------------------------- A_
@@ -188,7 +202,7 @@ __global__ void k_pack(const float *__restrict__ phi, uint32_t *__restrict__ bit
 // else r = (y - yb)/phisum; x_out_b = x_b + lambda * (r * phi_b).
 template <int MODE, bool ACC>
 __global__ void __launch_bounds__(256) k_proj_gap_vec(
-    const float *__restrict__ x, Mask<MODE> M, const float *__restrict__ y,
+    const float *__restrict__ x, ConstMask<MODE> M, const float *__restrict__ y,
     float *__restrict__ y1, const float *__restrict__ phisum, float *__restrict__ xo,
     float lam, int B, int64_t hw, double *__restrict__ rn) {
     const int64_t n4 = hw >> 2;
@@ -234,7 +248,7 @@ __global__ void __launch_bounds__(256) k_proj_gap_vec(
 }
 
 template <int MODE, bool ACC>
-__global__ void k_proj_gap_scalar(const float *__restrict__ x, Mask<MODE> M,
+__global__ void k_proj_gap_scalar(const float *__restrict__ x, ConstMask<MODE> M,
                                   const float *__restrict__ y, float *__restrict__ y1,
                                   const float *__restrict__ phisum, float *__restrict__ xo,
                                   float lam, int B, int64_t hw, double *__restrict__ rn) {
@@ -269,7 +283,7 @@ __global__ void k_proj_gap_scalar(const float *__restrict__ x, Mask<MODE> M,
 // update, so x crosses HBM once while registers stay low.
 template <int MODE, bool ACC>
 __global__ void __launch_bounds__(256) k_proj_gap_smem(
-    const float *__restrict__ x, Mask<MODE> M, const float *__restrict__ y,
+    const float *__restrict__ x, ConstMask<MODE> M, const float *__restrict__ y,
     float *__restrict__ y1, const float *__restrict__ phisum, float *__restrict__ xo,
     float lam, int B, int64_t hw, double *__restrict__ rn) {
     extern __shared__ float xs[];  // [B][blockDim.x]
@@ -306,7 +320,7 @@ __global__ void __launch_bounds__(256) k_proj_gap_smem(
 // [b][thread]), one HBM pass over theta and b.
 template <int MODE>
 __global__ void __launch_bounds__(128) k_proj_admm_smem(
-    const float *__restrict__ th, const float *__restrict__ bb, Mask<MODE> M,
+    const float *__restrict__ th, const float *__restrict__ bb, ConstMask<MODE> M,
     const float *__restrict__ y, const float *__restrict__ phisum, float *__restrict__ v,
     float *__restrict__ xo, float lam, float gamma, int B, int64_t hw, double *__restrict__ rn) {
     extern __shared__ float st[];  // [2][B][blockDim.x]: t, b
@@ -338,7 +352,7 @@ __global__ void __launch_bounds__(128) k_proj_admm_smem(
 }
 
 template <int MODE, bool ACC>
-static void launch_gap_smem(const float *x, Mask<MODE> M, const float *y, float *y1,
+static void launch_gap_smem(const float *x, ConstMask<MODE> M, const float *y, float *y1,
                             const float *ps, float *xo, float lam, int B, int64_t hw,
                             cudaStream_t s, double *rn) {
     const size_t smem = sizeof(float) * (size_t)B * 256;  // <= 32 KB for B <= 32
@@ -347,7 +361,7 @@ static void launch_gap_smem(const float *x, Mask<MODE> M, const float *y, float 
 }
 
 template <int MODE>
-static void launch_admm_smem(const float *th, const float *bb, Mask<MODE> M, const float *y,
+static void launch_admm_smem(const float *th, const float *bb, ConstMask<MODE> M, const float *y,
                              const float *ps, float *v, float *xo, float lam, float gamma, int B,
                              int64_t hw, cudaStream_t s, double *rn) {
     // 128 threads: 2 * B * 128 floats <= 32 KB of shared memory for B <= 32
@@ -365,7 +379,7 @@ static void launch_admm_smem(const float *th, const float *bb, Mask<MODE> M, con
 // 2048 x 24, 11.6 and 424 without a ground truth.  A pass of its own (k_sqerr)
 // reads x once more and is a launch: 4.5 and 165 us on top.
 template <int MODE, bool ACC, bool SQ>
-__global__ void __launch_bounds__(256) k_gap_resid_vec(
+__global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
     const float *x, Mask<MODE> M, const float *y, float *__restrict__ y1, const float *phisum,
     float *__restrict__ c, int B, int64_t hw, double *__restrict__ rn, double *__restrict__ zero,
     int nzero, int rev, const float *orig, double *__restrict__ sq) {
@@ -382,7 +396,7 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
         const int64_t p = (rev ? n4 - 1 - q : q) << 2;  // rev: bottom rows first
         const uint4 w = M.word4(p);
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
+#pragma unroll (SQ ? 4 : 8)
         for (int b = 0; b < B; ++b) {
             const float4 a = ld4(x + b * hw + p), m = M.at4(b, p, w);
             s.x = fmaf(a.x, m.x, s.x);
@@ -431,7 +445,7 @@ __global__ void __launch_bounds__(256) k_gap_resid_vec(
 // iteration 586 us, 455 without a ground truth; a pass of its own takes 165
 // and x stored for it about 50).
 template <bool FIRST, bool WANT_X, bool SQ>
-__global__ void __launch_bounds__(256) k_admm_resid_vec(
+__global__ void __launch_bounds__(256, 4) k_admm_resid_vec(
     const float *tp, Mask<1> M, const float *y, const float *phisum, float *__restrict__ rnew,
     float *__restrict__ xo, float lam, float gamma, int B, int64_t hw, double *__restrict__ rn,
     double *__restrict__ zero, int nzero, int rev, const float *orig, double *__restrict__ sq) {
@@ -495,7 +509,7 @@ __global__ void __launch_bounds__(256) k_admm_resid_vec(
 // v = x - b.  x written only when xo != nullptr.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_proj_admm_vec(
-    const float *__restrict__ th, const float *__restrict__ bb, Mask<MODE> M,
+    const float *__restrict__ th, const float *__restrict__ bb, ConstMask<MODE> M,
     const float *__restrict__ y, const float *__restrict__ phisum, float *__restrict__ v,
     float *__restrict__ xo, float lam, float gamma, int B, int64_t hw, double *__restrict__ rn) {
     const int64_t n4 = hw >> 2;
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(256) k_proj_admm_vec(
 
 template <int MODE>
 __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__restrict__ bb,
-                                   Mask<MODE> M, const float *__restrict__ y,
+                                   ConstMask<MODE> M, const float *__restrict__ y,
                                    const float *__restrict__ phisum, float *__restrict__ v,
                                    float *__restrict__ xo, float lam, float gamma, int B,
                                    int64_t hw, double *__restrict__ rn) {
@@ -586,8 +600,8 @@ __global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, i
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                x[k] = i + k < n ? a[i + k] : 0.f;
-                y[k] = i + k < n ? b[i + k] : 0.f;
+                x[k] = i + k < n ? ld1(a + i + k) : 0.f;
+                y[k] = i + k < n ? ld1(b + i + k) : 0.f;
             }
         }
 #pragma unroll
@@ -664,13 +678,13 @@ int proj_gap_rn(const float *x, const float *phi, const uint32_t *mask_bits, con
         if (e != SCI_ERR_UNSUPPORTED) return e;
     }
     if (mask_bits) {
-        Mask<1> M{mask_bits, hw};
+        ConstMask<1> M{mask_bits, hw};
         if (accelerate)
             launch_gap_smem<1, true>(x, M, y, y1, phisum, x_out, lambda, Bi, hw, s, rn);
         else
             launch_gap_smem<1, false>(x, M, y, y1, phisum, x_out, lambda, Bi, hw, s, rn);
     } else {
-        Mask<0> M{phi, hw};
+        ConstMask<0> M{phi, hw};
         LAUNCH_GAP(0, M);
     }
 #undef LAUNCH_GAP
@@ -790,10 +804,10 @@ int proj_admm_rn(const float *theta, const float *b, const float *phi,
         if (e != SCI_ERR_UNSUPPORTED) return e;
     }
     if (mask_bits) {
-        Mask<1> M{mask_bits, hw};
+        ConstMask<1> M{mask_bits, hw};
         launch_admm_smem<1>(theta, b, M, y, phisum, v, x_out, lambda, gamma, Bi, hw, s, rn);
     } else {
-        Mask<0> M{phi, hw};
+        ConstMask<0> M{phi, hw};
         if (vec)
             k_proj_admm_vec<0><<<grid_for(hw / 4, 256), 256, 0, s>>>(theta, b, M, y, phisum, v,
                                                                      x_out, lambda, gamma, Bi, hw,

@@ -582,7 +582,8 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 // 256 x 8 iteration (4.5 now: launch and reduction).  At 2048 x 2048 x 24 the
 // float64 pipe bounded it at 0.74 ms; now issue does at 0.165 ms, 4.9 TB/s of
 // the 805 MB it reads.
-template <bool VEC>
+// FEW: an element per thread, in float64.
+template <bool VEC, bool FEW>
 __global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, int64_t n,
                                                double *out) {
     grid_dep_wait();
@@ -590,7 +591,12 @@ __global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, i
     s.clear();
     double acc = 0.0;
     int turn = 0;
-    for (int64_t i = 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
+    if (FEW) {
+        const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+        const double e = i < n ? (double)a[i] - (double)b[i] : 0.0;
+        acc = e * e;
+    }
+    for (int64_t i = FEW ? n : 4 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
          i += 4 * (int64_t)gridDim.x * blockDim.x) {
         float x[4], y[4], d[4];
         if (VEC) {
@@ -609,7 +615,7 @@ __global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, i
         s.add4(x, y, d);
         if ((++turn & 7) == 0) acc += s.take();
     }
-    acc += s.take();
+    if (!FEW) acc += s.take();
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     __shared__ double red[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -914,13 +920,15 @@ int sci_proj_admm(const float *theta, const float *b, const float *phi,
 int sci_sqerr_accum(const float *a, const float *b, int64_t n, double *out, void *stream) {
     SCI_CHECK_ARG(a && b && out && n >= 0, "sci_sqerr_accum: bad argument");
     if (n == 0) return SCI_OK;
-    // at least two groups of four per thread, at most four blocks per SM
-    const int64_t want = (n + 2047) / 2048, most = (int64_t)kSMs * 4;
+    // at least two groups of four per thread, at most four blocks per SM; few
+    // elements: one per thread, in float64, whose chain is the shorter one
+    constexpr int64_t kFew = 1 << 15;
+    const int64_t want = n <= kFew ? (n + 255) / 256 : (n + 2047) / 2048, most = (int64_t)kSMs * 4;
     const dim3 g((unsigned)(want < most ? want : most));
-    if (n % 4 == 0 && aligned16(a) && aligned16(b))
-        SCI_CUDA(launch_dep(k_sqerr<true>, g, dim3(256), 0, as_stream(stream), a, b, n, out));
-    else
-        SCI_CUDA(launch_dep(k_sqerr<false>, g, dim3(256), 0, as_stream(stream), a, b, n, out));
+    const auto kernel = n <= kFew ? k_sqerr<false, true>
+                        : n % 4 == 0 && aligned16(a) && aligned16(b) ? k_sqerr<true, false>
+                                                                     : k_sqerr<false, false>;
+    SCI_CUDA(launch_dep(kernel, g, dim3(256), 0, as_stream(stream), a, b, n, out));
     SCI_LAUNCHED("k_sqerr");
     return SCI_OK;
 }

@@ -65,25 +65,13 @@ struct SquareSum {
     // the active lanes of a warp together.
     __device__ __forceinline__ void add4(const float (&x)[4], const float (&y)[4],
                                          const float (&d)[4]) {
-        // differences of 0 or of 1e-12 to 1e18: their bits less one, as
-        // unsigned, put 0 last; a vote, so that the float64 form is not
-        // issued under a predicate by every warp
-        unsigned most = 0u, least = ~0u;
+        // The largest difference is 0 or 1e-12 to 1e18: its square holds the
+        // words of all four (what the others' lose below 1e-45 is 2^-69 of it).
+        constexpr unsigned least = 0x2b8cbcccu, span = 0x5d5e0b6bu - least;  // 1e-12f, 1e18f
+        unsigned most = 0u;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const unsigned m = __float_as_uint(d[k]) & 0x7fffffffu;
-            most = max(most, m);
-            least = min(least, m - 1u);
-        }
-        const bool out = most > __float_as_uint(1e18f) || least < __float_as_uint(1e-12f);
-        if (__any_sync(__activemask(), out)) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double e = (double)x[k] - (double)y[k];
-                wide += e * e;
-            }
-            return;
-        }
+        for (int k = 0; k < 4; ++k) most = max(most, __float_as_uint(d[k]) & 0x7fffffffu);
+        const bool out = most != 0u && most - least > span;
         // x - y = d + dl exactly, (d + dl)^2 = d^2 + 2 d dl + dl^2: words t (of
         // d^2), m (about 2^-24 of it) and l (2^-48)
         f2 D[2], dl[2], t[2], m[2], l[2];
@@ -98,9 +86,19 @@ struct SquareSum {
             l[h].v = 0ull;
             rest |= __float_as_uint(lo(dl[h])) | __float_as_uint(hi(dl[h]));
         }
-        // values within a factor of two of each other differ exactly: a vote
-        // mostly leaves this out where the frames agree
-        if (__any_sync(__activemask(), (rest << 1) != 0u)) {
+        // Values within a factor of two of each other differ exactly: a vote
+        // mostly leaves the rest out where the frames agree, and the float64
+        // form, which would otherwise be issued under a predicate by every warp.
+        const unsigned lanes = __activemask();
+        if (__any_sync(lanes, out || (rest << 1) != 0u)) {
+            if (__any_sync(lanes, out)) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const double e = (double)x[k] - (double)y[k];
+                    wide += e * e;
+                }
+                return;
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 f2 pe, me;

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "sci_tv.cuh"
+#include "sci_tv_rule.cuh"
 
 namespace sci {
 namespace tv {
@@ -188,16 +189,16 @@ static int choose_lag() {
 }
 
 // The register-tile pass (sci_tv_tile.cuh) where it is the faster one
-// (tile_wins).  SCI_TV_TILE=0 leaves every call to the row pipelines, 1 takes
+// (sci_tv_rule.cuh).  SCI_TV_TILE=0 leaves every call to the row pipelines, 1 takes
 // tiles at every size; switches that shape the row pipelines (SCI_TV_SLIM=0,
 // SCI_TV_LAG, SCI_TV_R, SCI_TV_CPL, SCI_TV_ORDER, SCI_SLIM_MINB,
 // SCI_TV_FORM) leave it off too.
-static bool use_tiles(int64_t nf, int64_t H, int64_t W, bool slim) {
+static bool use_tiles(tv::Pipeline pipe, int64_t nf, int64_t H, int64_t W, int updates) {
     if (const char *e = getenv("SCI_TV_TILE")) return atoi(e) != 0;
     for (const char *k : {"SCI_TV_LAG", "SCI_TV_R", "SCI_TV_CPL", "SCI_TV_ORDER",
                           "SCI_SLIM_MINB", "SCI_TV_FORM"})
         if (getenv(k)) return false;
-    return tv::tile_wins(nf, H, W, slim);
+    return tv::tile_wins(pipe, nf, H, W, updates, tv::SMAX);
 }
 
 static int choose_cpl(int64_t W) {
@@ -309,8 +310,6 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
     // any row chunking: tvx_proj_supported answers for it
     const bool clip = slim_enabled() && ra.rule == RULE_CLIP && !resid && U <= SMAX &&
                       aligned_for(4);
-    SCI_CHECK_ARG(!ra.detector || use_tiles(nf, H, W, slim),
-                  "tv: the spectral on-load projection needs tiles");
     SCI_CHECK_ARG(!proj || ra.detector || slim || clip || !(ra.phi || ra.rule == RULE_CLIP),
                   "tv: this on-load projection needs the lean pass (aligned frames)");
     const int cpl = slim ? cpl_pick : ((proj || ra.rule != RULE_SKIMAGE) ? 4 : cpl_pick);
@@ -318,9 +317,14 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
                      ((reinterpret_cast<uintptr_t>(f) | reinterpret_cast<uintptr_t>(u) |
                        reinterpret_cast<uintptr_t>(resid)) % (4 * cpl) == 0);
     const int minb = slim_minb(cpl);
-    // windows on tiles: any rule-0 call without a row chunking or column width of the caller's; offsets in 32 bits
-    const bool tiles = slim_enabled() && ra.rule == RULE_SKIMAGE && force_R <= 0 &&
-                       fcpl == 0 && H * W < (int64_t(1) << 30) && use_tiles(nf, H, W, slim);
+    // windows on tiles: any rule-0 call without a row chunking or column width
+    // of the caller's; offsets in 32 bits.  The spectral projection has no other
+    // form: its caller asked tv_cassi_supported.
+    const Pipeline pipe = slim ? PIPE_LEAN : vec ? PIPE_VECTOR : PIPE_SCALAR;
+    const bool tiles = slim_enabled() && ra.rule == RULE_SKIMAGE && force_R <= 0 && fcpl == 0 &&
+                       H * W < (int64_t(1) << 30) &&
+                       (ra.detector || use_tiles(pipe, nf, H, W, U));
+    SCI_CHECK_ARG(!ra.detector || tiles, "tv: the spectral on-load projection needs tiles");
     const float *pin = nullptr;
     float *pbuf[2] = {w.pa, w.pb};
     int pi = 0;
@@ -451,7 +455,7 @@ int tv_launch_phi(const float *f, float *u, int64_t nf, int64_t H, int64_t W, in
 bool tv_cassi_supported(int64_t L, int64_t H, int64_t W, int K) {
     const char *e = getenv("SCI_FUSED_PROJ");
     return !(e && atoi(e) == 0) && slim_enabled() && K >= 2 && K <= tv::SMAX + 1 &&
-           H * W < (int64_t(1) << 30) && use_tiles(L, H, W, true);
+           H * W < (int64_t(1) << 30) && use_tiles(tv::PIPE_LEAN, L, H, W, K - 1);
 }
 
 // tv_launch_impl with x + lam (r[h, w + step b] phi[h, w]) applied as x is

@@ -941,8 +941,7 @@ __global__ void __launch_bounds__(WPB * 32, min_blocks<CPL>()) k_tv_fixup(Pass P
 }
 
 // Host launchers (one translation unit each, compiled in parallel).
-bool tile_wins(int64_t nf, int64_t H, int64_t W, bool slim);  // sci_tv_tile.cu
-void tile_geometry(Pass &P);
+void tile_geometry(Pass &P);  // sci_tv_tile.cu
 int tile_columns();
 int64_t tile_blocks(const Pass &P);
 void launch_clip(const Pass &P, int SG, int proj, cudaStream_t s);  // sci_tv_clip.cu

@@ -29,11 +29,6 @@ namespace sci {
 // bit 0: a bounded bulk-copy wait of the batched projection gave up
 __device__ unsigned int g_batch_status;
 
-int tv_launch(const float *f, float *u, float *resid, int64_t nf, int64_t H, int64_t W,
-              int64_t fs, float weight, float eps, int K, int *steps, double *energy_out,
-              void *workspace, size_t ws_bytes, cudaStream_t s, int force_R);
-size_t tv_workspace_bytes(int64_t nf, int64_t H, int64_t W, int K);
-
 namespace batch {
 
 // x0 = At(y / Phi_sum) for every item (the start point of the GAP loop).
@@ -198,7 +193,7 @@ __global__ void __launch_bounds__(tv::WPB * 32, 3) k_batch_tv(const Table *__res
 size_t r256(size_t b) { return (b + 255) & ~size_t(255); }
 
 struct Layout {
-    size_t table, xp, y1, energy, stop, tvscratch, total;
+    size_t table, xp, y1, energy, stop, total;
     std::vector<size_t> item_xp, item_y1, item_c, item_e, item_e1, item_stop;
 };
 
@@ -230,17 +225,13 @@ Layout layout(const sci_batch_item *items, int n, int K) {
         L.item_stop.push_back(off);
         off += r256(sizeof(int) * (size_t)items[i].B + sizeof(unsigned));
     }
-    L.tvscratch = off;
-    size_t tvmax = 0;  // autotuning scratch: the largest single-item TV workspace
-    for (int i = 0; i < n; ++i)
-        tvmax = std::max(tvmax, tv_workspace_bytes(items[i].B, items[i].H, items[i].W, K));
-    off += r256(tvmax);
     L.total = off;
     return L;
 }
 
 constexpr int kMinR = 8;  // least rows of a chunk
-constexpr size_t kWaitBytes = 3080;  // workspace of the wait selftest
+// Workspace that the wait selftest asks for, as it always has (it uses one word).
+constexpr size_t kWaitBytes = 3080;
 
 int check(const sci_batch_item *items, int n, int K) {
     SCI_CHECK_ARG(items && n >= 1 && n <= MAXI, "batch: 1..%d items (got %d)", MAXI, n);
@@ -415,7 +406,7 @@ __global__ void k_wait_selftest(const unsigned *count, unsigned polls) {
 }
 
 int wait_selftest(unsigned polls, unsigned *count, cudaStream_t s) {
-    SCI_CUDA(cudaMemsetAsync(count, 0, kWaitBytes, s));
+    SCI_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned), s));
     k_wait_selftest<<<1, 32, 0, s>>>(count, polls);
     SCI_LAUNCHED("k_wait_selftest");
     return SCI_OK;
@@ -443,7 +434,7 @@ int enqueue(const Table &T, Table *dT, const Layout &L, char *ws, int n, int ite
         // the items' stop decisions and tickets: a ticket counts the TV
         // tasks of an iteration and is reset by the last one, so it starts
         // at zero once per solve
-        SCI_CUDA(cudaMemsetAsync(ws + L.stop, 0, L.tvscratch - L.stop, s));
+        SCI_CUDA(cudaMemsetAsync(ws + L.stop, 0, L.total - L.stop, s));
         bool narrow = false;
         for (int i = 0; i < n; ++i)
             narrow = narrow || T.it[i].tvq[0].cpl == 2 || narrow_tail(T.it[i].tvq[0]);
@@ -455,7 +446,7 @@ int enqueue(const Table &T, Table *dT, const Layout &L, char *ws, int n, int ite
         }
         return SCI_OK;
     }
-    const size_t ebytes = L.tvscratch - L.energy;
+    const size_t ebytes = L.total - L.energy;
     // bulk-copy projection unless a mask is not 16-byte aligned (the other
     // planes are checked by check(); SCI_PROJ_TMA=0 selects the plain kernel)
     int maxB = 1;

@@ -88,10 +88,10 @@ __device__ __forceinline__ void run_item(const tv::Pass &P, int frame, int chunk
                 Q.nbands = 3;
                 Q.own = lo - (64 - P.hr);
             }
-            return srun_mode<S, 2, ENERGY, 1, 1, 1>(Q, frame, chunk, band, lane, G2);
+            return srun_mode<S, 2, ENERGY, 1>(Q, frame, chunk, band, lane, G2);
         }
     }
-    srun_mode<S, 4, ENERGY, 1, 1, 1>(P, frame, chunk, band, lane, G4);
+    srun_mode<S, 4, ENERGY, 1>(P, frame, chunk, band, lane, G4);
 }
 
 // The TV pass with S dual updates of one work item, or (FIX) its re-run with

@@ -943,10 +943,8 @@ __global__ void __launch_bounds__(WPB * 32, min_blocks<CPL>()) k_tv_fixup(Pass P
 // Host launchers (one translation unit each, compiled in parallel).
 void tile_geometry(Pass &P);  // sci_tv_tile.cu
 int tile_columns();
-int64_t tile_blocks(const Pass &P);
 void launch_clip(const Pass &P, int SG, int proj, cudaStream_t s);  // sci_tv_clip.cu
 int clip_resident_blocks();
-int tile_resident_blocks();
 void launch_tile(const Pass &P, bool pin, bool final_pass, int proj, cudaStream_t s);
 void launch_tile_fix(const Pass &P, bool pin, int proj, cudaStream_t s);
 void launch_main4_c4(const Pass &P, bool pin, bool final_pass, cudaStream_t s);

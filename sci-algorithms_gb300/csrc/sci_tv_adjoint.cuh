@@ -3,7 +3,7 @@
 // Per dual update k (last to first): with g_k = grad u_k, n_k = |g_k|,
 // r_k = 1 / (1 + tw n_k) and p_{k+1} = r_k (p_k - tau g_k):
 //   gbar_k = -tau r_k pbar_{k+1} - (tw r_k / n_k) <pbar_{k+1}, p_{k+1}> g_k
-//            (0 for the second term where n_k = 0)
+//            (0 for the second term where g_k = 0)
 //   ubar_k = -div gbar_k;  fbar += ubar_k;  pbar_k = r_k pbar_{k+1} + grad ubar_k
 // from pbar_U = grad xbar, fbar = xbar (u_U = f - div p_U with ubar_U = xbar).
 //
@@ -122,9 +122,10 @@ __device__ __forceinline__ void adjoint(const Adj &P, int frame, int tr, int tc,
                 f2 g1, g2;
                 grad(u, below, right, j, c, g1, g2);
                 const f2 s = fma2(g1, g1, mul2(g2, g2));
-                // |g| is 0 or at least 1.08e-19 (the root of the least
-                // normal number): the bound keeps 1 / |g| finite at 0, where
-                // it meets g = 0
+                // n is 0 or at least 1.08e-19 (the root of the least normal
+                // number). Below that |g| gives n = 0 and the bound stands for
+                // it: the second term is then 0 where g is, and else at most
+                // tw |pbar| |p|, as for any g
                 const float n0 = sqrt_approx(lo(s)), n1 = sqrt_approx(hi(s));
                 const f2 den = fma2(tw2, mk2(n0, n1), one2);
                 ri[j][c] = mk2(rcp_approx(lo(den)), rcp_approx(hi(den)));

@@ -6,8 +6,10 @@
 // bit-identical; what differs is the schedule.  The row pipeline marches a
 // warp down a chunk of rows through a chain of S dependent stages per row:
 // on a small frame that chain, not the work, is the time.  Here a block
-// holds a window of 32 C columns x 2 N NW rows (64 x 48 as launched): thread = C columns x 2 N
-// rows, f, u and p in registers for all updates, two block barriers per
+// holds a window of 32 C columns x 2 N NW rows -- 64 x 48, or 64 x 32 where
+// there are few -- thread = C columns x 2 N rows, f, u and p held by the thread
+// for all updates (the larger window, at 80 registers, spills 180 to 300 bytes
+// of them; more registers and fewer warps were slower), two block barriers per
 // update and no chain longer than one update.
 //
 //  * Pairs.  A packed f32x2 value holds rows j and j + N of a thread's
@@ -24,10 +26,11 @@
 //  * What bounds it: issue.  About 80 instructions a pixel and pass (4
 //    updates: 30 packed FP32, 8 MUFU, 5 shuffles, 14 register moves that
 //    pair scalar results), 53-60 % of the issue slots at 24 warps per SM, and
-//    1.38 times the pixels in halo.  256 x 256 x 8 in a solve: 9 us against 19
-//    for the row pipeline, 256 x 256 x 28 17 against 24, 512 x 512 x 10 21
-//    against 30; 8 x 2048 x 2048 takes 180 us against 123, so large frames
-//    keep the row pipeline (tile_wins).
+//    1.38 times the pixels in halo.  In a solve, against the row pipeline: 64 x
+//    32 windows (32 warps per SM) at 256 x 256 x 8 9 us against 19; 64 x 48 (24
+//    warps) at 256 x 256 x 28 17 against 24 and 512 x 512 x 10 21 against 30; 8
+//    x 2048 x 2048 takes 180 us against 123, so large frames keep the row
+//    pipeline (sci_tv_rule.cuh).
 //  * Stop test as in the row pipeline: per-frame float64 energies, the last
 //    block decides (k_tv_tile), a second launch of the same body with the
 //    shorter update count rewrites the frames that stop (k_tv_tile_fix).
@@ -45,6 +48,7 @@ constexpr int HALO = SMAX;
 
 template <int C, int N, int NW>
 struct Geo {
+    static_assert(C == 2, "loads, stores and exchanges are of two columns");
     static constexpr int COLS = 32 * C, ROWS = 2 * N * NW;
 };
 
@@ -106,7 +110,6 @@ struct Cells {
                                          float (&v)[C]) const {
         const char *p = reinterpret_cast<const char *>(plane + base), *q = p + o;
         if (SCALAR) {
-            static_assert(!SCALAR || C == 2, "scalars: two columns");
             // in this order: the two loads touch the same sectors, and a row's
             // lines leave L1 before a second sweep over the rows
             float a, b;
@@ -116,13 +119,8 @@ struct Cells {
             v[C - 1] = row_in && cols > 1 ? b : 0.f;
             return;
         }
-        if constexpr (C == 4) {
-            const float4 t = *reinterpret_cast<const float4 *>(q);
-            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-        } else {
-            const float2 t = *reinterpret_cast<const float2 *>(q);
-            v[0] = t.x, v[1] = t.y;
-        }
+        const float2 t = *reinterpret_cast<const float2 *>(q);
+        v[0] = t.x, v[1] = t.y;
         if (MODE != INSIDE) {
 #pragma unroll
             for (int c = 0; c < C; ++c) v[c] = row_in && cols > 0 ? v[c] : 0.f;
@@ -164,8 +162,6 @@ struct Cells {
 #pragma unroll
                     for (int c = 0; c < C; ++c)
                         if (c < cols) q[c] = a[c];
-                } else if constexpr (C == 4) {
-                    *reinterpret_cast<float4 *>(q) = make_float4(a[0], a[1], a[2], a[3]);
                 } else {
                     *reinterpret_cast<float2 *>(q) = make_float2(a[0], a[1]);
                 }
@@ -237,20 +233,12 @@ struct Exchange {
     float v[NW][32 * C];
     __device__ __forceinline__ void put(int w, int lane, const float (&x)[C]) {
         float *p = &v[w][lane * C];
-        if constexpr (C == 4)
-            *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
-        else
-            *reinterpret_cast<float2 *>(p) = make_float2(x[0], x[1]);
+        *reinterpret_cast<float2 *>(p) = make_float2(x[0], x[1]);
     }
     __device__ __forceinline__ void get(int w, int lane, float (&x)[C]) const {
         const float *p = &v[w][lane * C];
-        if constexpr (C == 4) {
-            const float4 t = *reinterpret_cast<const float4 *>(p);
-            x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
-        } else {
-            const float2 t = *reinterpret_cast<const float2 *>(p);
-            x[0] = t.x, x[1] = t.y;
-        }
+        const float2 t = *reinterpret_cast<const float2 *>(p);
+        x[0] = t.x, x[1] = t.y;
     }
 };
 

@@ -16,7 +16,7 @@
 // reverse pass runs the adjoint of every TV step:
 //   p_{k+1} = (p_k - tau g_k) r_k,  r_k = 1 / (1 + (tau/w) n_k),  n_k = |g_k|,
 //   gbar_k = -tau r_k pbar_{k+1} - (tau/w) r_k (g_k / n_k) <pbar_{k+1}, p_{k+1}>
-//            (0 for the second term where n_k = 0: the safe-norm convention),
+//            (0 for the second term where g_k = 0: the safe-norm convention),
 //   ubar_k = -div gbar_k,  fbar += ubar_k,  pbar_k = r_k pbar_{k+1} + grad ubar_k.
 // then the adjoint of the projection (including d/dPhi through A, At and
 // Phi_sum, and d/dlambda_k), and finally of the measurement and x^0.
@@ -432,9 +432,9 @@ bool stored_tape(int64_t N, int64_t B, int64_t H, int64_t W, int K, int T) {
 // Frames whose tape the reverse pass recomputes and consumes at a time: the
 // tape stays in L2 (it is overwritten there by the next frames' and never
 // needed in HBM) as long as it is small against the 129 MB, and a launch
-// should fill the GPU.  Measured at 16 x 256 x 256 x 8 (2.9 MB of tape a
-// frame), forward and reverse pass: 16 frames at a time 6.91 ms, 24 6.95, 32
-// 7.01, 48 7.14, 64 7.17, all 128 7.45.
+// should fill the GPU.  Measured at one shape, 16 x 256 x 256 x 8 (2.9 MB of
+// tape a frame), forward and reverse pass: 16 frames at a time, fewest of those
+// tried, 6.91 ms, 24 6.95, 32 7.01, 48 7.14, 64 7.17, all 128 7.45.
 int64_t tape_frames(int64_t nf, int64_t hw, int U) {
     const int64_t frame = 4 * hw * (3 * U - 1);
     const int64_t l2 = (40 << 20) / frame, fill = (1 << 20) / hw;

@@ -193,12 +193,12 @@ static int choose_lag() {
 // tiles at every size; switches that shape the row pipelines (SCI_TV_SLIM=0,
 // SCI_TV_LAG, SCI_TV_R, SCI_TV_CPL, SCI_TV_ORDER, SCI_SLIM_MINB,
 // SCI_TV_FORM) leave it off too.
-static bool use_tiles(tv::Pipeline pipe, int64_t nf, int64_t H, int64_t W, int updates) {
+static bool tiles_if(bool faster) {
     if (const char *e = getenv("SCI_TV_TILE")) return atoi(e) != 0;
     for (const char *k : {"SCI_TV_LAG", "SCI_TV_R", "SCI_TV_CPL", "SCI_TV_ORDER",
                           "SCI_SLIM_MINB", "SCI_TV_FORM"})
         if (getenv(k)) return false;
-    return tv::tile_wins(pipe, nf, H, W, updates, tv::SMAX);
+    return faster;
 }
 
 static int choose_cpl(int64_t W) {
@@ -320,10 +320,13 @@ static int tv_launch_core(const float *f, float *u, float *resid, int64_t nf, in
     // windows on tiles: any rule-0 call without a row chunking or column width
     // of the caller's; offsets in 32 bits.  The spectral projection has no other
     // form: its caller asked tv_cassi_supported.
-    const Pipeline pipe = slim ? PIPE_LEAN : vec ? PIPE_VECTOR : PIPE_SCALAR;
+    const Pipeline pipe = slim                          ? PIPE_LEAN
+                          : vec                         ? PIPE_VECTOR
+                          : aligned_for(tile_columns()) ? PIPE_PAIRS
+                                                        : PIPE_SCALAR;
     const bool tiles = slim_enabled() && ra.rule == RULE_SKIMAGE && force_R <= 0 && fcpl == 0 &&
                        H * W < (int64_t(1) << 30) &&
-                       (ra.detector || use_tiles(pipe, nf, H, W, U));
+                       (ra.detector || tiles_if(tile_wins(pipe, nf, H, W, U, SMAX)));
     SCI_CHECK_ARG(!ra.detector || tiles, "tv: the spectral on-load projection needs tiles");
     const float *pin = nullptr;
     float *pbuf[2] = {w.pa, w.pb};
@@ -455,7 +458,7 @@ int tv_launch_phi(const float *f, float *u, int64_t nf, int64_t H, int64_t W, in
 bool tv_cassi_supported(int64_t L, int64_t H, int64_t W, int K) {
     const char *e = getenv("SCI_FUSED_PROJ");
     return !(e && atoi(e) == 0) && slim_enabled() && K >= 2 && K <= tv::SMAX + 1 &&
-           H * W < (int64_t(1) << 30) && use_tiles(tv::PIPE_LEAN, L, H, W, K - 1);
+           H * W < (int64_t(1) << 30) && tiles_if(tv::spectral_tile_wins(L, H, W, K - 1));
 }
 
 // tv_launch_impl with x + lam (r[h, w + step b] phi[h, w]) applied as x is

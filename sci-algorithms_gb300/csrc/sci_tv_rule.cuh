@@ -23,7 +23,8 @@
 //     updates 16 x 1024 x 1024 99.8 / 106 and 110 / 129, an iteration of ADMM
 //     with 24 such frames 273 / 261 (11856);
 //   generic, other rows: 1 update 6 x 1023 x 1025 24.6 / 22.7 (2964); 4 updates
-//     16 x 1001 x 1023 112 / 134 (7600), 32 x 1001 x 1023 211 / 203 (15200);
+//     16 x 1001 x 1023 112 / 134 (7600), 32 x 1001 x 1023 211 / 203 (15200); of 4 k
+//     + 2 columns 17 x 1508 x 1090 (12920), an iteration of a solve 211 / 242;
 //   several passes, aligned: 30 steps of 22 x 1024 x 1024 1085 / 1235 (10868), of
 //     36 x 1024 x 1024 9 steps 468 / 447 (17784).
 #pragma once
@@ -41,16 +42,19 @@ inline int64_t rule_count(int64_t n, int64_t width) {
     return n <= width ? 1 : 1 + (n - width + own - 1) / own;
 }
 
-// The pipeline that would run the call instead.
-enum Pipeline { PIPE_LEAN = 0, PIPE_VECTOR = 1, PIPE_SCALAR = 2 };
+// The pipeline that would run the call instead: lean; generic with vector
+// loads; generic with scalar loads, as tiles too; generic with scalar loads where
+// tiles load pairs (rows of 4 k + 2 columns, wider than 512).
+enum Pipeline { PIPE_LEAN = 0, PIPE_VECTOR = 1, PIPE_SCALAR = 2, PIPE_PAIRS = 3 };
 
 // The most windows for `updates` dual updates in all, up to `most` a pass.
 inline int64_t tile_line(Pipeline pipe, int64_t W, int updates, int most) {
     // one pass of 1, 2, 3, 4 updates, several passes; W <= 256, <= 512, wider
-    static const int line[3][3][5] = {
+    static const int line[4][3][5] = {
         {{600, 605, 1290, 4500, 0}, {585, 585, 1330, 3400, 0}, {290, 580, 790, 2500, 0}},
         {{600, 1200, 4500, 5900, 11000}, {585, 4400, 14000, 14000, 14000}, {530, 990, 7950, 7950, 14000}},
-        {{900, 1290, 3390, 5900, 7950}, {900, 2500, 4400, 6000, 14000}, {1330, 1490, 10900, 10900, 14000}}};
+        {{900, 1290, 3390, 5900, 7950}, {900, 2500, 4400, 6000, 14000}, {1330, 1490, 10900, 10900, 14000}},
+        {{1850, 14000, 14000, 14000, 14000}, {1850, 14000, 14000, 14000, 14000}, {1850, 14000, 14000, 14000, 14000}}};
     const int w = W <= 256 ? 0 : W <= 512 ? 1 : 2;
     if (updates <= most) return line[pipe][w][updates - 1];
     // a last pass of one update, which wide aligned rows take better on the
@@ -69,6 +73,20 @@ inline bool tile_wins(Pipeline pipe, int64_t nf, int64_t H, int64_t W, int updat
     // 23 frames 45.5 / 45.6 us, 74 134 / 105)
     if (n > 3000 && 2 * rows * (kWinRows - 2 * kWinHalo) > 3 * H) return false;
     return n <= tile_line(pipe, W, updates, most);
+}
+
+// Whether a spectral solve of L bands runs its TV (1 to 4 updates) on tiles that
+// apply the projection as they load x: that saves the projection kernel's pass
+// too, so it pays for more windows. Measured, us an iteration with / without,
+// 256 x 256 x 28 (980 windows): 1 update 15.9 / 16.1, 2 20.5 / 23.2, 4 23.8 /
+// 28.0; 2 updates 512 x 512 x 28 (3276) 49.8 / 50.4, 700 x 700 x 8 (1872) 30.7 /
+// 31.8, 300 x 700 x 28 (2912) 42.0 / 40.0. Rows the lean pass cannot take gain
+// more: 511 x 513 x 28 (3640) 59.2 / 62.9.
+inline bool spectral_tile_wins(int64_t L, int64_t H, int64_t W, int updates) {
+    static const int line[3][4] = {{2100, 2100, 2100, 4500}, {3300, 3300, 3300, 3300}, {2500, 1900, 2500, 2500}};
+    const int w = W <= 256 ? 0 : W <= 512 ? 1 : 2;
+    const bool lean = W % (w == 2 ? 4 : 2) == 0;
+    return L * rule_count(H, kWinRows) * rule_count(W, kWinCols) <= line[w][lean ? updates - 1 : 3];
 }
 
 }  // namespace tv

@@ -7,7 +7,8 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                     "sci-algorithms_gb300", "csrc")
-LEAN, VECTOR, SCALAR = 0, 1, 2  # lean pass; generic, rows aligned for vectors; other rows
+# lean pass; generic, rows aligned for vectors; other rows; rows of 4 k + 2 columns
+LEAN, VECTOR, SCALAR, PAIRS = 0, 1, 2, 3
 
 # (pipeline, frames, H, W, dual updates, us on the row pipeline, us on tiles):
 # for each pipeline, width and number of updates the largest call measured that
@@ -117,7 +118,9 @@ int main() {
     int pipe, updates;
     long long nf, H, W;
     while (std::scanf("%d %lld %lld %lld %d", &pipe, &nf, &H, &W, &updates) == 5)
-        std::printf("%d\n", (int)sci::tv::tile_wins((sci::tv::Pipeline)pipe, nf, H, W, updates, 4));
+        std::printf("%d\n", (int)(pipe < 0
+            ? sci::tv::spectral_tile_wins(nf, H, W, updates)
+            : sci::tv::tile_wins((sci::tv::Pipeline)pipe, nf, H, W, updates, 4)));
 }
 """
 
@@ -157,3 +160,32 @@ def test_calls_near_the_lines_take_the_faster_pass(decide):
     (SCALAR, 6, 1023, 1025, 1), (SCALAR, 5, 2047, 2049, 1), (SCALAR, 30, 49, 4097, 3)])
 def test_calls_that_tiles_slowed_down(decide, pipe, nf, H, W, updates):
     assert decide([(pipe, nf, H, W, updates)]) == [False]
+
+
+# Rows that tiles load in pairs and the pipeline one by one: tiles to the end of
+# the range measured (us on the row pipeline, on tiles).
+@pytest.mark.parametrize("nf,H,W,updates,pipe_us,tile_us", [
+    (17, 1508, 1090, 4, 241.6, 211.2),
+    (28, 1024, 1026, 3, 182.9, 152.8),
+    (28, 1024, 1026, 4, 190.0, 170.6),
+    (28, 1024, 1026, 8, 469.2, 368.1),
+    (28, 1024, 1026, 19, 1244.8, 954.6),
+    (18, 1508, 1090, 3, 186.4, 151.3),
+    (18, 1508, 1090, 4, 192.8, 168.6),
+    (18, 1508, 1090, 8, 475.8, 365.2),
+    (18, 1508, 1090, 19, 1260.9, 947.1),
+    (1, 1080, 1922, 1, 14.3, 11.4),
+    (1, 1080, 1922, 2, 23.8, 17.9)])
+def test_rows_of_pairs_stay_on_tiles(decide, nf, H, W, updates, pipe_us, tile_us):
+    assert tile_us < pipe_us
+    assert decide([(PAIRS, nf, H, W, updates)]) == [True]
+
+
+# Spectral solves, projection on load or not: (bands, H, W, updates, us an
+# iteration without, with).
+@pytest.mark.parametrize("L,H,W,updates,apart,fused", [
+    (28, 256, 256, 1, 16.1, 15.9), (28, 256, 256, 2, 23.2, 20.5), (28, 256, 256, 4, 28.0, 23.8),
+    (20, 511, 300, 2, 27.7, 27.5), (16, 512, 512, 3, 40.7, 33.8), (16, 511, 513, 2, 46.8, 37.3),
+    (8, 512, 800, 4, 37.4, 31.9), (28, 300, 700, 2, 40.0, 42.0), (28, 512, 800, 2, 67.8, 76.1)])
+def test_spectral_solves_take_the_faster_form(decide, L, H, W, updates, apart, fused):
+    assert decide([(-1, L, H, W, updates)]) == [fused < apart]

@@ -32,8 +32,8 @@
 //  * Sums: the squared error (sci_sqerr.cuh) and 1 - SSIM are accumulated
 //    with compensated float32 additions over 8 rows and then added to float64.
 //
-// Measured at 2048 x 2048 x 8: 0.205 ms for the kernel (3.4 ms in float64),
-// 0.18 of it without the squared error's third word and the windows' range
+// Measured at 2048 x 2048 x 8: 0.202 ms for the kernel (3.4 ms in float64),
+// 0.184 of it without the squared error's third word and the windows' range
 // check; the packed float32 arithmetic of the windows bounds it (no spills at
 // 3 blocks per SM; 4 blocks spill).  Against float64 (rms over frames, this
 // kernel / float64 quotients of float32 moments): mean SSIM at noise 0.003 2e-12

@@ -375,9 +375,10 @@ static void launch_admm_smem(const float *th, const float *bb, ConstMask<MODE> M
 // c = (y - yb)/phisum.  The x update x + lambda (c phi_b) is applied by the
 // TV kernel while it loads x (same arithmetic as k_proj_gap).
 // SQ: also adds sum (orig - x)^2 to *sq, the squared error of the iteration
-// that produced x: 16.0 us an iteration at 256 x 256 x 8 and 568 at 2048 x
-// 2048 x 24, 11.6 and 424 without a ground truth.  A pass of its own (k_sqerr)
-// reads x once more and is a launch: 4.5 and 165 us on top.
+// that produced x: 15.9 us an iteration at 256 x 256 x 8 and 541 at 2048 x
+// 2048 x 24, 11.3 and 422 without a ground truth.  A pass of its own (k_sqerr)
+// reads x once more and is a launch: 4.4 and 160 us on top.  Four blocks per
+// SM, with some spills where SQ: left to itself the compiler took three, 562 us.
 template <int MODE, bool ACC, bool SQ>
 __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
     const float *x, Mask<MODE> M, const float *y, float *__restrict__ y1, const float *phisum,
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
 // yb = sum_b phi_b t_b and r_{k+1} = (y - yb) / (phisum + gamma).  With xo
 // it also writes x = t + lambda (r phi_b) of every frame (a second sweep).
 // SQ: also adds sum (orig - x)^2 to *sq, x stored or not (2048 x 2048 x 24: an
-// iteration 586 us, 455 without a ground truth; a pass of its own takes 165
+// iteration 583 us, 452 without a ground truth; a pass of its own takes 160
 // and x stored for it about 50).
 template <bool FIRST, bool WANT_X, bool SQ>
 __global__ void __launch_bounds__(256, 4) k_admm_resid_vec(
@@ -579,8 +580,8 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 // *out += sum (a - b)^2, the PSNR numerator of an iteration.  Few blocks: each
 // ends in one float64 atomic on the same word, and 2048 of them, with two
 // conversions and two float64 operations per element, were 12 us of a 256 x
-// 256 x 8 iteration (4.5 now: launch and reduction).  At 2048 x 2048 x 24 the
-// float64 pipe bounded it at 0.74 ms; now issue does at 0.165 ms, 4.9 TB/s of
+// 256 x 8 iteration (4.4 now: launch and reduction).  At 2048 x 2048 x 24 the
+// float64 pipe bounded it at 0.74 ms; now issue does at 0.160 ms, 5.0 TB/s of
 // the 805 MB it reads.
 // FEW: an element per thread, in float64.
 template <bool VEC, bool FEW>
@@ -921,7 +922,8 @@ int sci_sqerr_accum(const float *a, const float *b, int64_t n, double *out, void
     SCI_CHECK_ARG(a && b && out && n >= 0, "sci_sqerr_accum: bad argument");
     if (n == 0) return SCI_OK;
     // at least two groups of four per thread, at most four blocks per SM; few
-    // elements: one per thread, in float64, whose chain is the shorter one
+    // elements: one per thread, in float64, whose chain is the shorter one (32768
+    // elements 1.9 us against 3.1, 131072 4.6 against 3.2)
     constexpr int64_t kFew = 1 << 15;
     const int64_t want = n <= kFew ? (n + 255) / 256 : (n + 2047) / 2048, most = (int64_t)kSMs * 4;
     const dim3 g((unsigned)(want < most ? want : most));

@@ -15,7 +15,7 @@
 //
 // What bounds it: issue, about 90 instructions for four elements (60 where
 // the vote below finds the differences exact).  k_sqerr at 2048 x 2048 x 8 and
-// x 24: 57 and 165 us (two words 47 and 136, float64 254 and 742).
+// x 24: 55 and 160 us (two words 47 and 136, float64 254 and 742).
 #pragma once
 
 #include "sci_common.cuh"

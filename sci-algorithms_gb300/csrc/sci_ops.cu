@@ -375,10 +375,10 @@ static void launch_admm_smem(const float *th, const float *bb, ConstMask<MODE> M
 // c = (y - yb)/phisum.  The x update x + lambda (c phi_b) is applied by the
 // TV kernel while it loads x (same arithmetic as k_proj_gap).
 // SQ: also adds sum (orig - x)^2 to *sq, the squared error of the iteration
-// that produced x: 15.9 us an iteration at 256 x 256 x 8 and 541 at 2048 x
+// that produced x: 16.0 us an iteration at 256 x 256 x 8 and 533 at 2048 x
 // 2048 x 24, 11.3 and 422 without a ground truth.  A pass of its own (k_sqerr)
-// reads x once more and is a launch: 4.4 and 160 us on top.  Four blocks per
-// SM, with some spills where SQ: left to itself the compiler took three, 562 us.
+// reads x once more and is a launch: 4.5 and 148 us on top.  Four blocks per
+// SM, with some spills where SQ: three, as the compiler chose, cost 20 us more.
 template <int MODE, bool ACC, bool SQ>
 __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
     const float *x, Mask<MODE> M, const float *y, float *__restrict__ y1, const float *phisum,
@@ -392,6 +392,7 @@ __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
     double racc = 0.0, sacc = 0.0;
     SquareSum se;
     se.clear();
+    int held = 0;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n4;
          q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = (rev ? n4 - 1 - q : q) << 2;  // rev: bottom rows first
@@ -405,9 +406,11 @@ __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
             s.z = fmaf(a.z, m.z, s.z);
             s.w = fmaf(a.w, m.w, s.w);
             if (SQ) se.add4(ld4(orig + b * hw + p), a);
-            if (SQ && (b & 7) == 7) sacc += se.take();
+            if (SQ && ++held == SquareSum::kMost) {
+                sacc += se.take();
+                held = 0;
+            }
         }
-        if (SQ) sacc += se.take();
         const float4 yv = ld4(y + p), ps = ld4(phisum + p);
         float4 r;
         if (ACC) {
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
     if (rn) rn_flush(racc, rn);
     if (SQ) {
         if (rn) __syncthreads();
-        rn_flush(sacc, sq);
+        rn_flush(sacc + se.take(), sq);
     }
 }
 
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(256, 4) k_gap_resid_vec(
 // yb = sum_b phi_b t_b and r_{k+1} = (y - yb) / (phisum + gamma).  With xo
 // it also writes x = t + lambda (r phi_b) of every frame (a second sweep).
 // SQ: also adds sum (orig - x)^2 to *sq, x stored or not (2048 x 2048 x 24: an
-// iteration 583 us, 452 without a ground truth; a pass of its own takes 160
+// iteration 579 us, 452 without a ground truth; a pass of its own takes 148
 // and x stored for it about 50).
 template <bool FIRST, bool WANT_X, bool SQ>
 __global__ void __launch_bounds__(256, 4) k_admm_resid_vec(
@@ -462,6 +465,7 @@ __global__ void __launch_bounds__(256, 4) k_admm_resid_vec(
     double racc = 0.0, sacc = 0.0;
     SquareSum se;
     se.clear();
+    int held = 0;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n4;
          q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = (rev ? n4 - 1 - q : q) << 2;
@@ -493,15 +497,17 @@ __global__ void __launch_bounds__(256, 4) k_admm_resid_vec(
                                 fmaf(lam, r.z * m.z, t.z), fmaf(lam, r.w * m.w, t.w));
                 if (WANT_X) st4(xo + b * hw + p, xv);
                 if (SQ) se.add4(ld4(orig + b * hw + p), xv);
-                if (SQ && (b & 7) == 7) sacc += se.take();
+                if (SQ && ++held == SquareSum::kMost) {
+                    sacc += se.take();
+                    held = 0;
+                }
             }
-            if (SQ) sacc += se.take();
         }
     }
     if (rn) rn_flush(racc, rn);
     if (SQ) {
         if (rn) __syncthreads();
-        rn_flush(sacc, sq);
+        rn_flush(sacc + se.take(), sq);
     }
 }
 
@@ -580,8 +586,8 @@ __global__ void k_proj_admm_scalar(const float *__restrict__ th, const float *__
 // *out += sum (a - b)^2, the PSNR numerator of an iteration.  Few blocks: each
 // ends in one float64 atomic on the same word, and 2048 of them, with two
 // conversions and two float64 operations per element, were 12 us of a 256 x
-// 256 x 8 iteration (4.4 now: launch and reduction).  At 2048 x 2048 x 24 the
-// float64 pipe bounded it at 0.74 ms; now issue does at 0.160 ms, 5.0 TB/s of
+// 256 x 8 iteration (4.5 now: launch and reduction).  At 2048 x 2048 x 24 the
+// float64 pipe bounded it at 0.74 ms; now issue does at 0.148 ms, 5.4 TB/s of
 // the 805 MB it reads.
 // FEW: an element per thread, in float64.
 template <bool VEC, bool FEW>
@@ -614,7 +620,7 @@ __global__ void __launch_bounds__(256) k_sqerr(const float *a, const float *b, i
 #pragma unroll
         for (int k = 0; k < 4; ++k) d[k] = x[k] - y[k];
         s.add4(x, y, d);
-        if ((++turn & 7) == 0) acc += s.take();
+        if (++turn % SquareSum::kMost == 0) acc += s.take();
     }
     if (!FEW) acc += s.take();
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

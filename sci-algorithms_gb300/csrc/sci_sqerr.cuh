@@ -15,7 +15,7 @@
 //
 // What bounds it: issue, about 90 instructions for four elements (60 where
 // the vote below finds the differences exact).  k_sqerr at 2048 x 2048 x 8 and
-// x 24: 55 and 160 us (two words 47 and 136, float64 254 and 742).
+// x 24: 52 and 148 us (two words 47 and 136, float64 254 and 742).
 #pragma once
 
 #include "sci_common.cuh"
@@ -55,6 +55,11 @@ __device__ __forceinline__ f2 two_mul(f2 a, f2 b, f2 &err) {
 }
 
 struct SquareSum {
+    // Calls of add4 between two of take() at most: a word then holds 128 squares
+    // of at most 1e36.  take() is a dozen float64 operations, 16 clocks of the
+    // SM's float64 pipe each and warp: with one for 8 calls k_sqerr took 160 us
+    // at 2048 x 2048 x 24 instead of 148.
+    static constexpr int kMost = 64;
     f2 s0, s1, s2;  // sum of the even and the odd elements, in three words
     double wide;
     __device__ __forceinline__ void clear() {

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) k_mse(const float *__restrict__ a,
                                           gscale * (x.z - y.z), gscale * (x.w - y.w)));
         } else {
             se.add4(x, y);
-            if (++held == 8) {
+            if (++held == SquareSum::kMost) {
                 acc += se.take();
                 held = 0;
             }
